@@ -113,23 +113,20 @@ struct gdn_cuda_handle {
 	double *yacc = nullptr; // FP32_REFINE: FP64 solution of the transport solve
 	float *rhs = nullptr; // FP32_REFINE: residual, right-hand side of the corrections
 	int refine_passes = 1;
-	int kin_mode = 1; // 1: a launch per sweep level, 2: one cooperative launch per sweep, 3: flag-driven,
-	                  // 4: spatial parts
+	int kin_mode = 1; // 1: a launch per sweep level, 2: one cooperative launch per sweep, 3: row-driven,
+	                  // 4: row-driven by spatial parts
 	bool kin_autotune = true; // pick kin_mode at attach by timing the modes
 	int kin_grid[3] = {0, 0, 0}; // CTAs of the cooperative sweep, per accumulate mode
-	int kin_fgrid[3] = {0, 0, 0}; // CTAs of the flag-driven sweep, per accumulate mode
-	int2 *kchunks = nullptr; // [nchunks] level-aligned 32-item chunks (first item, end item)
-	int nchunks = 0;
-	int *kready = nullptr; // [nitems] readiness flags of the flag-driven sweep
-	unsigned *kqueue = nullptr; // its chunk counter
+	int kin_fgrid[3] = {0, 0, 0}; // CTAs of the row-driven sweep that fit at once, per accumulate mode
+	int2 *kgroups = nullptr; // [ngroups] level-aligned groups of a CTA's items (first item, end item)
+	int ngroups = 0;
 	long long spin_limit = 1LL << 21; // polls of a bounded device-side wait (~1 s)
-	// the spatial-parts sweep: item list by part, level-aligned chunks, chunk ranges per part
+	// the spatial-parts sweep: item list by part, level-aligned groups, group ranges per part
 	int *plist = nullptr;
-	int2 *pchunks = nullptr;
-	int *part_chunk_off = nullptr;
+	int2 *pgroups = nullptr;
+	int *part_group_off = nullptr;
 	int nparts = 0;
-	int kin_pgrid[3] = {0, 0, 0}; // CTAs of the parts sweep that fit at once, per accumulate mode
-	int max_chunks = 1; // most 32-item chunks in one level
+	int max_groups = 1; // most groups in one level
 	int *level_off_dev = nullptr;
 	unsigned *bar = nullptr; // [2] grid barrier of the cooperative sweep
 	int *err = nullptr; // set on the device when a barrier wait gave up
@@ -658,20 +655,19 @@ static int attach_impl(gdn_cuda_handle *h, const gdn_cuda_mesh *m, const gdn_cud
 		GDN_TRY(dalloc(h, &h->err, 1));
 		GDN_CUDA_TRY(cudaMemsetAsync(h->bar, 0, 2 * sizeof(unsigned), s));
 		GDN_CUDA_TRY(cudaMemsetAsync(h->err, 0, sizeof(int), s));
-		// the flag-driven sweep: level-aligned chunks in sweep order
-		std::vector<int2> chunks;
+		// the row-driven sweep: level-aligned groups in sweep order
+		const int gi = kin_group_items(fp64);
+		std::vector<int2> groups;
 		for (int l = 0; l < nl; l++) {
-			const int nch = (h->level_off[l + 1] - h->level_off[l] + 31) / 32;
-			h->max_chunks = nch > h->max_chunks ? nch : h->max_chunks;
-			for (int k0 = h->level_off[l]; k0 < h->level_off[l + 1]; k0 += 32)
-				chunks.push_back(make_int2(k0, k0 + 32 < h->level_off[l + 1] ? k0 + 32 : h->level_off[l + 1]));
+			const int end = h->level_off[l + 1], ng = (end - h->level_off[l] + gi - 1) / gi;
+			h->max_groups = ng > h->max_groups ? ng : h->max_groups;
+			for (int k0 = h->level_off[l]; k0 < end; k0 += gi)
+				groups.push_back(make_int2(k0, k0 + gi < end ? k0 + gi : end));
 		}
-		h->nchunks = (int)chunks.size();
-		GDN_TRY(dalloc(h, &h->kchunks, chunks.size()));
-		GDN_CUDA_TRY(cudaMemcpyAsync(h->kchunks, chunks.data(), chunks.size() * sizeof(int2), cudaMemcpyHostToDevice,
+		h->ngroups = (int)groups.size();
+		GDN_TRY(dalloc(h, &h->kgroups, groups.size()));
+		GDN_CUDA_TRY(cudaMemcpyAsync(h->kgroups, groups.data(), groups.size() * sizeof(int2), cudaMemcpyHostToDevice,
 									 s));
-		GDN_TRY(dalloc(h, &h->kready, nu));
-		GDN_TRY(dalloc(h, &h->kqueue, 1));
 		GDN_TRY(kin_prepare_grids(h));
 		GDN_TRY(kin_prepare_parts(h, m));
 		GDN_CUDA_TRY(cudaStreamSynchronize(s));
@@ -994,7 +990,7 @@ static int kin_sweeps(gdn_cuda_handle *h, const void *f, int acc, int bdata, lon
 	p.nv = h->nv;
 	const int nl = (int)h->level_off.size() - 1;
 	if (h->kin_mode == 2) {
-		int grid = h->kin_grid[acc] < h->max_chunks ? h->kin_grid[acc] : h->max_chunks;
+		int grid = h->kin_grid[acc] < h->max_groups ? h->kin_grid[acc] : h->max_groups;
 		grid = grid > 0 ? grid : 1;
 		p.item_begin = 0;
 		p.item_end = h->level_off[nl];
@@ -1003,21 +999,14 @@ static int kin_sweeps(gdn_cuda_handle *h, const void *f, int acc, int bdata, lon
 		nlaunch++;
 		return GDN_CUDA_OK;
 	}
-	if (h->kin_mode == 4) {
+	if (h->kin_mode >= 3) {
+		const bool parts = h->kin_mode == 4;
+		const int grid = parts ? h->nparts : (h->kin_fgrid[acc] < h->ngroups ? h->kin_fgrid[acc] : h->ngroups);
 		p.item_begin = 0;
 		p.item_end = h->level_off[nl];
-		GDN_TRY((launch_kin_parts<F, Y, T>(p, h->plist, h->pchunks, h->part_chunk_off, h->nparts, h->kready,
-										   h->ne * h->nv, h->err, h->spin_limit, acc, bdata, h->rk3_sparse,
-										   h->stream)));
-		nlaunch++;
-		return GDN_CUDA_OK;
-	}
-	if (h->kin_mode == 3) {
-		p.item_begin = 0;
-		p.item_end = h->level_off[nl];
-		GDN_TRY((launch_kin_flags<F, Y, T>(p, h->kchunks, h->nchunks, h->kin_fgrid[acc] > 0 ? h->kin_fgrid[acc] : 1,
-										   h->kqueue, h->kready, h->ne * h->nv, h->err, h->spin_limit, acc, bdata,
-										   h->rk3_sparse, h->stream)));
+		GDN_TRY((launch_kin_flow<F, Y, T>(p, parts ? h->pgroups : h->kgroups, h->ngroups, parts ? h->plist : nullptr,
+										  parts ? h->part_group_off : nullptr, grid > 0 ? grid : 1, h->ne * h->nv, h->err,
+										  h->spin_limit, acc, bdata, h->rk3_sparse, h->stream)));
 		nlaunch++;
 		return GDN_CUDA_OK;
 	}
@@ -1100,42 +1089,28 @@ static int kin_enqueue(gdn_cuda_handle *h, long long &nlaunch)
 	return GDN_CUDA_OK;
 }
 
-// CTAs of the cooperative and the flag-driven sweeps for the variants this
+// CTAs of the cooperative and the row-driven sweeps for the variants this
 // handle's precision runs
-static int kin_prepare_flag_grids(gdn_cuda_handle *h)
+static int kin_prepare_flow_grids(gdn_cuda_handle *h)
 {
 	const int sp = h->rk3_sparse;
 	switch (h->precision) {
 	case GDN_CUDA_FP64:
-		return kin_flags_grid<double, double, double>(h->device, 0, sp, &h->kin_fgrid[0]);
+		return kin_flow_grid<double, double, double>(h->device, 0, sp, &h->kin_fgrid[0]);
 	case GDN_CUDA_FP32:
-		return kin_flags_grid<float, float, float>(h->device, 0, sp, &h->kin_fgrid[0]);
+		return kin_flow_grid<float, float, float>(h->device, 0, sp, &h->kin_fgrid[0]);
 	case GDN_CUDA_BF16_STORE:
-		return kin_flags_grid<__nv_bfloat16, float, float>(h->device, 0, sp, &h->kin_fgrid[0]);
+		return kin_flow_grid<__nv_bfloat16, float, float>(h->device, 0, sp, &h->kin_fgrid[0]);
 	default:
-		GDN_TRY((kin_flags_grid<double, float, float>(h->device, 1, sp, &h->kin_fgrid[1])));
-		return kin_flags_grid<float, float, float>(h->device, 2, sp, &h->kin_fgrid[2]);
+		GDN_TRY((kin_flow_grid<double, float, float>(h->device, 1, sp, &h->kin_fgrid[1])));
+		return kin_flow_grid<float, float, float>(h->device, 2, sp, &h->kin_fgrid[2]);
 	}
 }
 
 static int kin_prepare_grids(gdn_cuda_handle *h)
 {
 	const int sp = h->rk3_sparse;
-	GDN_TRY(kin_prepare_flag_grids(h));
-	switch (h->precision) {
-	case GDN_CUDA_FP64:
-		GDN_TRY((kin_parts_grid<double, double, double>(h->device, 0, sp, &h->kin_pgrid[0])));
-		break;
-	case GDN_CUDA_FP32:
-		GDN_TRY((kin_parts_grid<float, float, float>(h->device, 0, sp, &h->kin_pgrid[0])));
-		break;
-	case GDN_CUDA_BF16_STORE:
-		GDN_TRY((kin_parts_grid<__nv_bfloat16, float, float>(h->device, 0, sp, &h->kin_pgrid[0])));
-		break;
-	default:
-		GDN_TRY((kin_parts_grid<double, float, float>(h->device, 1, sp, &h->kin_pgrid[1])));
-		GDN_TRY((kin_parts_grid<float, float, float>(h->device, 2, sp, &h->kin_pgrid[2])));
-	}
+	GDN_TRY(kin_prepare_flow_grids(h));
 	switch (h->precision) {
 	case GDN_CUDA_FP64:
 		return kin_levels_grid<double, double, double>(h->device, 0, sp, &h->kin_grid[0]);
@@ -1151,14 +1126,14 @@ static int kin_prepare_grids(gdn_cuda_handle *h)
 
 // The spatial parts of the parts sweep: as many parts as CTAs of every
 // launched variant fit at once (at least 32 elements each), the item list by
-// part (device), its level-aligned chunks (at most 32 items) and each part's
-// chunk range.
+// part (device), its level-aligned groups (at most a CTA's items) and each
+// part's group range.
 static int kin_prepare_parts(gdn_cuda_handle *h, const gdn_cuda_mesh *m)
 {
 	int cap = 0;
 	for (int a = 0; a < 3; a++)
-		if (h->kin_pgrid[a] > 0)
-			cap = cap == 0 || h->kin_pgrid[a] < cap ? h->kin_pgrid[a] : cap;
+		if (h->kin_fgrid[a] > 0)
+			cap = cap == 0 || h->kin_fgrid[a] < cap ? h->kin_fgrid[a] : cap;
 	const long long byelem = h->ne / 32 > 0 ? h->ne / 32 : 1;
 	h->nparts = (int)(cap < byelem ? cap : byelem);
 	if (h->nparts < 1)
@@ -1172,14 +1147,15 @@ static int kin_prepare_parts(gdn_cuda_handle *h, const gdn_cuda_mesh *m)
 	const long long nitems = h->ne * h->nv;
 	GDN_TRY(dalloc(h, &h->plist, nitems));
 	std::vector<int> plist, pkey;
-	GDN_TRY(kin_build_parts(h->e2q, h->node, h->ne, lo, hi, h->items, nitems, h->nv, h->nparts, h->rnb, h->rpm,
+	GDN_TRY(kin_build_parts(h->e2q, h->node, h->ne, lo, hi, h->items, nitems, h->nv, h->nparts,
 							h->plist, plist, pkey, h->stream));
 	h->launches += 5;
-	std::vector<int2> chunks;
+	const int gi = kin_group_items(h->precision == GDN_CUDA_FP64);
+	std::vector<int2> groups;
 	std::vector<int> off(h->nparts + 1, 0);
 	long long i = 0;
 	for (int b = 0; b < h->nparts; b++) {
-		off[b] = (int)chunks.size();
+		off[b] = (int)groups.size();
 		size_t l = 0; // level of the current item (plist is in sweep order within a part)
 		int start = -1, cnt = 0;
 		size_t lstart = 0;
@@ -1187,9 +1163,9 @@ static int kin_prepare_parts(gdn_cuda_handle *h, const gdn_cuda_mesh *m)
 			const int k = plist[i];
 			while (l + 1 < h->level_off.size() && k >= h->level_off[l + 1])
 				l++;
-			if (start < 0 || l != lstart || cnt == 32) {
+			if (start < 0 || l != lstart || cnt == gi) {
 				if (start >= 0)
-					chunks.push_back(make_int2(start, cnt));
+					groups.push_back(make_int2(start, start + cnt));
 				start = (int)i;
 				cnt = 0;
 				lstart = l;
@@ -1197,14 +1173,14 @@ static int kin_prepare_parts(gdn_cuda_handle *h, const gdn_cuda_mesh *m)
 			cnt++;
 		}
 		if (start >= 0)
-			chunks.push_back(make_int2(start, cnt));
+			groups.push_back(make_int2(start, start + cnt));
 	}
-	off[h->nparts] = (int)chunks.size();
-	GDN_TRY(dalloc(h, &h->pchunks, chunks.size()));
-	GDN_TRY(dalloc(h, &h->part_chunk_off, off.size()));
-	GDN_CUDA_TRY(cudaMemcpyAsync(h->pchunks, chunks.data(), chunks.size() * sizeof(int2), cudaMemcpyHostToDevice,
+	off[h->nparts] = (int)groups.size();
+	GDN_TRY(dalloc(h, &h->pgroups, groups.size()));
+	GDN_TRY(dalloc(h, &h->part_group_off, off.size()));
+	GDN_CUDA_TRY(cudaMemcpyAsync(h->pgroups, groups.data(), groups.size() * sizeof(int2), cudaMemcpyHostToDevice,
 								 h->stream));
-	GDN_CUDA_TRY(cudaMemcpyAsync(h->part_chunk_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice,
+	GDN_CUDA_TRY(cudaMemcpyAsync(h->part_group_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice,
 								 h->stream));
 	GDN_CUDA_TRY(cudaStreamSynchronize(h->stream));
 	return GDN_CUDA_OK;

@@ -78,7 +78,7 @@ struct KinSweepParams {
 	const void *f; // right-hand side of M1 y = f (F)
 	void *y; // solution, written level by level; read back as the inflow traces (Y)
 	double *yacc; // refinement: FP64 solution, = y (ACC 1) or += y (ACC 2)
-	const void *G; // [k][10][10] inverse of the M1 diagonal block (T)
+	const void *G; // [k][10][10] inverse of the M1 diagonal block, by columns (T)
 	const void *rs; // [k][4] own-side v.vn per face (T)
 	const void *rcoef; // [k] theta dt / det (T)
 	const int4 *rnb; // [k] per face: inflow neighbour item, -(bf + 1) inflow boundary face, INT_MIN none
@@ -104,33 +104,28 @@ int launch_kin_levels(const KinSweepParams &p, const int *level_off, int nlevels
 template <typename F, typename Y, typename T>
 int kin_levels_grid(int device, int acc, int sparse, int *grid);
 
-// The same solve driven by per-item readiness flags in one launch: CTAs take
-// level-aligned 32-item chunks (chunks[c] = first item, end item) in sweep
-// order from *queue and wait only for their items' upwind neighbours' flags
-// (ready[nitems], cleared with *queue before the launch); a wait that gives
-// up after spin_limit polls sets *err.
-template <typename F, typename Y, typename T>
-int launch_kin_flags(const KinSweepParams &p, const int2 *chunks, int nchunks, int grid, unsigned *queue, int *ready,
-					 long long nitems, int *err, long long spin_limit, int acc, int bdata, int sparse, cudaStream_t s);
-template <typename F, typename Y, typename T>
-int kin_flags_grid(int device, int acc, int sparse, int *grid);
+// items a CTA of the sweeps takes at once (five per warp); the groups of the
+// row-driven sweep hold at most as many
+int kin_group_items(int fp64);
 
-// The same solve with each CTA of one cooperative launch sweeping one compact
-// spatial part in sweep order (plist, level-aligned chunks pchunks[c] = first
-// list position and count, part b's chunks from part_chunk_off[b]); only
-// upwind items of other parts (bit 28 of their face's rpm entry) are waited
-// for through ready[] (cleared before the launch).
+// The same solve in one cooperative launch driven by the solution rows
+// themselves: every word of y is marked unwritten (all bits set) first, then
+// CTAs walk level-aligned
+// groups of items (groups[g] = first item, end item) in sweep order, and a
+// warp waits until the traces of its items are written.  CTA b takes the groups
+// b, b + grid, ..., or with `group_off` those of its own spatial part (positions in
+// list[]).  A wait that gives up after spin_limit polls sets *err.
 template <typename F, typename Y, typename T>
-int launch_kin_parts(const KinSweepParams &p, const int *plist, const int2 *pchunks, const int *part_chunk_off,
-					 int nparts, int *ready, long long nitems, int *err, long long spin_limit, int acc, int bdata,
-					 int sparse, cudaStream_t s);
+int launch_kin_flow(const KinSweepParams &p, const int2 *groups, int ngroups, const int *list, const int *group_off,
+					int grid, long long nitems, int *err, long long spin_limit, int acc, int bdata, int sparse,
+					cudaStream_t s);
 template <typename F, typename Y, typename T>
-int kin_parts_grid(int device, int acc, int sparse, int *grid);
+int kin_flow_grid(int device, int acc, int sparse, int *grid);
 // the parts: elements split into nparts equal ranges along a Morton curve of
 // their centroids (bounding box lo, hi); plist (device) and its host copy,
-// the part of every list entry (host), bit 28 of rpm set for external inflow
+// the part of every list entry (host)
 int kin_build_parts(const int *e2q, const double *node, long long ne, const double lo[3], const double hi[3],
-					const int *items, long long nitems, int nv, int nparts, const int4 *rnb, int4 *rpm, int *plist,
+					const int *items, long long nitems, int nv, int nparts, int *plist,
 					std::vector<int> &plist_host, std::vector<int> &pkey_host, cudaStream_t s);
 
 // Level schedule of the upwind item graph on the device (Kahn's algorithm by

@@ -391,10 +391,12 @@ __global__ void __launch_bounds__(kBlkThreads, 4)
 		atomicMax(bad, 1);
 		return;
 	}
-	GT *Gk = G + kk * 100 + posn * 10;
+	// by columns (entry (i, j) at 10 j + i): the sweep takes rows in pairs, and
+	// the item's ten lanes write one contiguous column at a time
+	GT *Gk = G + kk * 100 + posn;
 #pragma unroll
 	for (int t = 0; t < 10; t++)
-		Gk[(col >> (4 * t)) & 15] = (GT)a[10 + t];
+		Gk[((col >> (4 * t)) & 15) * 10] = (GT)a[10 + t];
 }
 
 // per-item records of the sweep
@@ -557,219 +559,372 @@ __device__ __forceinline__ void store10(S *p, const T v[10])
 	}
 }
 
-// One level of the block forward substitution.  A CTA takes 32 consecutive
-// items of the level with 6 warps: lane = item, warp = field, so the tables
-// are warp-uniform (constant-bank operands) and every thread owns one field
-// of one item end to end:
-//   traces of the inflow faces (24 independent loads, one round trip),
+// Block forward substitution, a warp per five items.  Six lanes serve an item,
+// one per field c (lanes 30 and 31 idle):
 //   t = sum_inflow s E_f S tr_f,  r = f - coef Minv t,  y = G r.
-// G of the 32 items is staged by cp.async into shared memory while the
-// traces are in flight; its per-item stride (100 floats / 102 doubles) keeps
-// the 16-byte row reads conflict-free.  Levels are launched with programmatic
-// stream serialization: level l + 1 stages G, records and f while level l
-// runs, and waits (griddepcontrol.wait) only before its trace loads.
-constexpr int kSwItems = 32;
-constexpr int kSwThreads = 6 * 32;
+// The sweep's limit is the memory instructions of an item, not its arithmetic:
+// with lane = item every access of a warp touched 32 items 240 bytes apart, 32
+// L1 lookups per instruction, and a level of 14 k items took ~7 us on lookups
+// alone.  Here every global access moves 16-byte pieces of an item's
+// contiguous 240-byte (FP32) rows, six lanes side by side:
+//   stage   G and f of the item into shared memory (cp.async), its records
+//           into registers (data no sweep step writes);
+//   wait    the caller waits for the item's upwind neighbours;
+//   solve   the whole row of each inflow neighbour (at most three faces: sum s
+//           = 0) into shared memory through L2, one round trip; the face
+//           permutation then picks the traces out of the row there; y leaves
+//           through shared memory in the same 16-byte pieces.
+// G is read by its six lanes at one address (broadcast), one wavefront per
+// 16 bytes; a warp shares nothing with other warps, so there is no CTA barrier.
+// ms per step before (lane = item, 32 items per CTA) and after, the fastest
+// grouping of each (jittered meshes, d3q4): 17^3 FP64 0.76 / 0.45, 24^3 FP32 with
+// one refinement 3.03 / 1.47, 40^3 FP64 2.83 / 1.89, 64^3 FP32 5.83 / 3.62; a
+// level of 457 items takes 2.6 us (4.4 before), of 9250 items 3.5 us (7.4).
+constexpr int kSwSlots = 5; // items per warp
 
+// Warps per CTA (static shared memory below 48 KB) and items per CTA.
 template <typename T>
-struct SweepG {
-	static constexpr int stride = sizeof(T) == 4 ? 100 : 102;
-	typedef typename std::conditional<sizeof(T) == 4, float4, double2>::type vec;
-	static constexpr int per_vec = 16 / sizeof(T);
+struct SweepCfg {
+	static constexpr int warps = sizeof(T) == 4 ? 4 : 3;
+	static constexpr int threads = 32 * warps;
+	static constexpr int items = kSwSlots * warps;
+	// G row stride: the five items' 16-byte reads in distinct banks
+	static constexpr int gstride = sizeof(T) == 4 ? 100 : 102;
+};
+int kin_group_items(int fp64)
+{
+	return fp64 ? SweepCfg<double>::items : SweepCfg<float>::items;
+}
+
+template <typename F, typename T>
+struct alignas(16) SweepWarp {
+	T G[kSwSlots * SweepCfg<T>::gstride];
+	T tr[kSwSlots * 180]; // per item: three neighbour rows [6][10]; then its y
+	F f[kSwSlots * 60];
 };
 
-// A chunk: up to 32 items of one level, [k0, min(k0 + 32, item_end)), or with
-// `list` the items list[k0 .. item_end).  Lane = item, warp = field c.  It is
-// processed in three pieces:
-//   chunk_stage_G  G of the chunk's items into shared memory (cp.async, one
-//                  commit group);
-//   chunk_load     the thread's records, right-hand side and FP64
-//                  accumulator into registers (data no sweep step writes);
-//   chunk_solve    traces of the upwind neighbours, t = sum_inflow s E S tr,
-//                  r = f - coef Minv t, then (after its G group has landed and
-//                  a barrier) y = G r and the stores, and a closing barrier.
-// Between chunk_load and chunk_solve the caller waits for the upwind items the
-// chunk depends on.  L2 = true reads the traces through L2 only (L1 is not
-// coherent with other SMs' writes made during the same launch); FENCE = true
-// orders every thread's y stores device-wide before the closing barrier;
-// WAITG = cp.async groups committed after this chunk's G (0 or 1).
 template <typename T, int ACC>
-struct ChunkIn {
+struct SweepLane {
 	long long k;
-	int nloc;
+	int slot, c;
 	bool act;
 	int nbk[4], pmk[4];
-	T fv[10];
-	double ya[ACC == 2 ? 10 : 1];
-	T coef;
-	T s[4];
-	int v;
+	unsigned inflow; // faces with a trace
+	T s[4], coef;
+	double2 ya[ACC == 2 ? 5 : 1];
 };
 
-__device__ __forceinline__ int chunk_nloc(long long k0, long long item_end)
+// nloc (1 to 5) items k0 .. k0 + nloc - 1, or with `list` list[k0 ..].
+template <typename F, typename T, int ACC, bool BD>
+__device__ __forceinline__ void warp_stage(const KinSweepParams &p, long long k0, int nloc, const int *list,
+										   SweepWarp<F, T> &sh, SweepLane<T, ACC> &in)
 {
-	const long long rem = item_end - k0;
-	return rem < kSwItems ? (int)rem : kSwItems;
-}
-
-template <typename T>
-__device__ __forceinline__ void chunk_stage_G(const KinSweepParams &p, long long k0, int nloc, const int *list, T *gsh)
-{
-	typedef SweepG<T> SG;
-	constexpr int VPC = SG::per_vec, CH = 100 / VPC;
-	const T *G = reinterpret_cast<const T *>(p.G);
-	for (int q = threadIdx.x; q < nloc * CH; q += kSwThreads) {
-		const int it = q / CH, ch = q - it * CH;
-		const long long kit = list ? (long long)list[k0 + it] : k0 + it;
-		__pipeline_memcpy_async(gsh + it * SG::stride + ch * VPC, G + kit * 100 + ch * VPC, 16);
+	constexpr int GV = 16 / sizeof(T), GP = 100 / GV;
+	constexpr int FB = 60 * sizeof(F) % 16 == 0 ? 16 : 8, FV = FB / sizeof(F), FP = 60 / FV;
+	const int lane = threadIdx.x & 31;
+	const int slot = lane < 30 ? lane / 6 : kSwSlots - 1, c = lane - 6 * (lane / 6);
+	in.slot = slot;
+	in.c = c;
+	in.act = lane < 30 && slot < nloc;
+	const long long kk = k0 + (in.act ? slot : 0);
+	const long long k = list ? (long long)list[kk] : kk;
+	in.k = k;
+	if (in.act) {
+		const T *G = reinterpret_cast<const T *>(p.G) + k * 100;
+		const F *f = reinterpret_cast<const F *>(p.f) + k * 60;
+#pragma unroll
+		for (int i = 0; i < (GP + 5) / 6; i++)
+			if (c + 6 * i < GP)
+				__pipeline_memcpy_async(sh.G + slot * SweepCfg<T>::gstride + (c + 6 * i) * GV, G + (c + 6 * i) * GV, 16);
+#pragma unroll
+		for (int i = 0; i < (FP + 5) / 6; i++)
+			if (c + 6 * i < FP)
+				__pipeline_memcpy_async(sh.f + slot * 60 + (c + 6 * i) * FV, f + (c + 6 * i) * FV, FB);
 	}
 	__pipeline_commit();
-}
-
-template <typename F, typename T, int ACC, bool BD>
-__device__ __forceinline__ void chunk_load(const KinSweepParams &p, long long k0, long long item_end, const int *list,
-										   ChunkIn<T, ACC> &in)
-{
-	const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
-	in.nloc = chunk_nloc(k0, item_end);
-	in.act = lane < in.nloc;
-	const long long k = list ? (long long)list[k0 + (in.act ? lane : 0)] : k0 + (in.act ? lane : 0);
-	in.k = k;
 	const int4 nb4 = p.rnb[k];
 	const int4 pm4 = p.rpm[k];
 	in.nbk[0] = nb4.x, in.nbk[1] = nb4.y, in.nbk[2] = nb4.z, in.nbk[3] = nb4.w;
 	in.pmk[0] = pm4.x, in.pmk[1] = pm4.y, in.pmk[2] = pm4.z, in.pmk[3] = pm4.w;
-	load10<F, T>(reinterpret_cast<const F *>(p.f) + k * 60 + c * 10, in.fv);
-	if (ACC == 2)
-		load10<double, double>(p.yacc + k * 60 + c * 10, in.ya);
 	in.coef = reinterpret_cast<const T *>(p.rcoef)[k];
 	const T *rs = reinterpret_cast<const T *>(p.rs) + k * 4;
 #pragma unroll
 	for (int f = 0; f < 4; f++)
 		in.s[f] = rs[f];
-	in.v = BD ? p.items[k] % p.nv : 0;
+	if (ACC == 2) {
+		const double2 *ya = reinterpret_cast<const double2 *>(p.yacc + k * 60);
+#pragma unroll
+		for (int i = 0; i < 5; i++)
+			in.ya[i] = ya[c + 6 * i];
+	}
+	in.inflow = 0;
+#pragma unroll
+	for (int f = 0; f < 4; f++)
+		if (in.nbk[f] >= 0 || (BD && in.nbk[f] != INT_MIN))
+			in.inflow |= 1u << f;
+	if (!in.act)
+		in.inflow = 0;
+	if (BD) { // boundary inflow faces: f_eq of the data, in face order
+#pragma unroll
+		for (int f = 0; f < 4; f++)
+			if ((in.inflow >> f & 1) && in.nbk[f] < 0) {
+				const int r = __popc(in.inflow & ((1u << f) - 1));
+				const int v = p.items[k] % p.nv;
+				const double *b = p.bt + (((long long)(-in.nbk[f] - 1) * p.nv + v) * 6 + c) * 6;
+#pragma unroll
+				for (int jj = 0; jj < 6; jj++)
+					sh.tr[slot * 180 + r * 60 + c * 10 + jj] = (T)b[jj];
+				in.pmk[f] = 0x543210;
+			}
+	}
 }
 
-template <typename F, typename Y, typename T, int ACC, bool BD, bool SPARSE, bool L2, bool FENCE, int WAITG>
-__device__ __forceinline__ void chunk_solve(const KinSweepParams &p, const ChunkIn<T, ACC> &in, T *gsh)
+// y = G r with G by columns; FP32 in packed row pairs
+template <typename T>
+__device__ __forceinline__ void block_product(const T *G, const T r[10], T y[10])
 {
-	typedef SweepG<T> SG;
-	const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
-	const Tables<T> &tb = tab<T>();
-	const long long k = in.k;
-	T r[10];
-	{
-		T tr[4][6];
 #pragma unroll
-		for (int f = 0; f < 4; f++) {
-			const int nbv = in.nbk[f];
-			if (nbv >= 0) {
-				const Y *yn = reinterpret_cast<const Y *>(p.y) + (long long)nbv * 60 + c * 10;
+	for (int i = 0; i < 10; i++)
+		y[i] = T(0);
+	const double2 *g = reinterpret_cast<const double2 *>(G);
 #pragma unroll
-				for (int jj = 0; jj < 6; jj++) {
-					const Y *q = yn + ((in.pmk[f] >> (4 * jj)) & 15);
-					tr[f][jj] = (T)(L2 ? Store<Y>::load_l2(q) : Store<Y>::load(q));
-				}
-			} else if (BD && nbv != INT_MIN) {
-				const double *b = p.bt + (((long long)(-nbv - 1) * p.nv + in.v) * 6 + c) * 6;
+	for (int q = 0; q < 50; q++) {
+		const double2 gv = g[q];
+		y[2 * q % 10] += gv.x * r[2 * q / 10];
+		y[2 * q % 10 + 1] += gv.y * r[2 * q / 10];
+	}
+}
+template <>
+__device__ __forceinline__ void block_product<float>(const float *G, const float r[10], float y[10])
+{
+	float2 acc[5];
 #pragma unroll
-				for (int jj = 0; jj < 6; jj++)
-					tr[f][jj] = (T)b[jj];
-			} else {
+	for (int i = 0; i < 5; i++)
+		acc[i] = make_float2(0.f, 0.f);
+	const float4 *g = reinterpret_cast<const float4 *>(G);
 #pragma unroll
-				for (int jj = 0; jj < 6; jj++)
-					tr[f][jj] = T(0);
-			}
+	for (int q = 0; q < 25; q++) {
+		const float4 gv = g[q];
+		const int a = 4 * q, b = 4 * q + 2;
+		acc[a % 10 / 2] = __ffma2_rn(make_float2(gv.x, gv.y), make_float2(r[a / 10], r[a / 10]), acc[a % 10 / 2]);
+		acc[b % 10 / 2] = __ffma2_rn(make_float2(gv.z, gv.w), make_float2(r[b / 10], r[b / 10]), acc[b % 10 / 2]);
+	}
+#pragma unroll
+	for (int i = 0; i < 5; i++) {
+		y[2 * i] = acc[i].x;
+		y[2 * i + 1] = acc[i].y;
+	}
+}
+
+// "Not written yet" in the solution array of the row-driven sweeps: all bits
+// set, a NaN that no arithmetic returns (for FP64 the upper word decides).
+__device__ __forceinline__ bool unwritten(float v)
+{
+	return __float_as_uint(v) == 0xffffffffu;
+}
+__device__ __forceinline__ bool unwritten(double v)
+{
+	return (unsigned)__double2hiint(v) == 0xffffffffu;
+}
+__device__ __forceinline__ float written(float v)
+{
+	return unwritten(v) ? __uint_as_float(0x7fffffffu) : v;
+}
+__device__ __forceinline__ double written(double v)
+{
+	return unwritten(v) ? __hiloint2double(0x7fffffff, -1) : v;
+}
+
+// the neighbour item of the r-th inflow face (-1: none, or a boundary face)
+template <typename T, int ACC>
+__device__ __forceinline__ void inflow_rows(const SweepLane<T, ACC> &in, int nr[3])
+{
+	nr[0] = nr[1] = nr[2] = -1;
+	int cnt = 0;
+#pragma unroll
+	for (int f = 0; f < 4; f++)
+		if (in.inflow >> f & 1) {
+			const int n = in.nbk[f] >= 0 ? in.nbk[f] : -1;
+			nr[0] = cnt == 0 ? n : nr[0];
+			nr[1] = cnt == 1 ? n : nr[1];
+			nr[2] = cnt == 2 ? n : nr[2];
+			cnt++;
 		}
-		// t_i = sum over the faces through node i of s_f (S tr_f)_ii
+}
+
+// The inflow neighbours' whole rows into shared memory (through L2: L1 is not
+// coherent with other SMs' writes made during the launch), then the lane's
+// traces x[f] (undefined on faces without inflow).  Call after warp_stage.
+template <typename F, typename T, int ACC>
+__device__ __forceinline__ void warp_gather(const KinSweepParams &p, const SweepLane<T, ACC> &in, const int nr[3],
+											SweepWarp<F, T> &sh, T x[4][6])
+{
+	constexpr int YV = 16 / sizeof(T), YP = 60 / YV;
+	T *tr0 = sh.tr + in.slot * 180;
+	const T *y = reinterpret_cast<const T *>(p.y);
+#pragma unroll
+	for (int r = 0; r < 3; r++)
+		if (nr[r] >= 0) {
+			const T *row = y + (long long)nr[r] * 60;
+#pragma unroll
+			for (int i = 0; i < (YP + 5) / 6; i++)
+				if (in.c + 6 * i < YP)
+					__pipeline_memcpy_async(tr0 + r * 60 + (in.c + 6 * i) * YV, row + (in.c + 6 * i) * YV, 16);
+		}
+	__pipeline_commit();
+	__pipeline_wait_prior(0);
+	__syncwarp();
+#pragma unroll
+	for (int f = 0; f < 4; f++)
+		if (in.inflow >> f & 1) {
+			const T *row = tr0 + __popc(in.inflow & ((1u << f) - 1)) * 60 + in.c * 10;
+#pragma unroll
+			for (int jj = 0; jj < 6; jj++)
+				x[f][jj] = row[(in.pmk[f] >> (4 * jj)) & 15];
+		}
+}
+
+// Row-driven wait and gather: the rows are their own readiness flags.  Every
+// word of y is "unwritten" when the solve starts, and a trace is ready when it
+// is not: no flags, fences or ordering between an item's words are needed.
+// The rows are fetched at once; if a trace is missing, one lane per row polls
+// the row's last word, and the rows are fetched again when all have arrived.
+// false when *err is set, or after spin_limit polls (then *err is set here),
+// so a lost producer ends the launch instead of hanging it.
+template <typename F, typename T, int ACC>
+__device__ __forceinline__ bool warp_gather_wait(const KinSweepParams &p, const SweepLane<T, ACC> &in, const int nr[3],
+												 SweepWarp<F, T> &sh, T x[4][6], int *err, long long spin_limit)
+{
+	const int mine = in.c == 0 ? nr[0] : (in.c == 1 ? nr[1] : (in.c == 2 ? nr[2] : -1));
+	const unsigned *last = reinterpret_cast<const unsigned *>(reinterpret_cast<const T *>(p.y) +
+															   (long long)(mine >= 0 ? mine : 0) * 60 + 60) - 1;
+	for (long long it = 0;; it++) {
+		warp_gather<F, T, ACC>(p, in, nr, sh, x);
+		bool missing = false;
+#pragma unroll
+		for (int f = 0; f < 4; f++)
+			if (in.inflow >> f & 1) {
+#pragma unroll
+				for (int jj = 0; jj < 6; jj++)
+					missing |= unwritten(x[f][jj]);
+			}
+		if (!__any_sync(0xffffffffu, missing))
+			return true;
+		for (;; it++) {
+			if ((it & 63) == 63 && __any_sync(0xffffffffu, *(const volatile int *)err != 0))
+				return false;
+			if (it >= spin_limit) {
+				if ((threadIdx.x & 31) == 0)
+					atomicExch(err, 1);
+				return false;
+			}
+			unsigned v = 0;
+			if (mine >= 0)
+				asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(last) : "memory");
+			if (!__any_sync(0xffffffffu, v == 0xffffffffu))
+				break;
+		}
+	}
+}
+
+// After the gather: solve, y (and the FP64 accumulator) stored.
+// SPARSE: the tables have the P2 structural zeros; FLOW: row-driven sweep.  The
+// products are the plain sums over the tables: their symmetric forms
+// (lift_minv_sym) cancel more, and cost FP32 sweeps a factor two in error.
+template <typename F, typename T, int ACC, bool SPARSE, bool FLOW>
+__device__ __forceinline__ void warp_solve(const KinSweepParams &p, const SweepLane<T, ACC> &in, const T x[4][6],
+										   SweepWarp<F, T> &sh)
+{
+	constexpr int YV = 16 / sizeof(T), YP = 60 / YV;
+	const Tables<T> &tb = tab<T>();
+	const int slot = in.slot, c = in.c;
+	T *tr0 = sh.tr + slot * 180;
+	T y[10];
+	{
+		// t_i = sum over the inflow faces through node i of s_f (S tr_f)_ii
 		T t[10];
 #pragma unroll
 		for (int i = 0; i < 10; i++)
 			t[i] = T(0);
 #pragma unroll
-		for (int f = 0; f < 4; f++) {
+		for (int f = 0; f < 4; f++)
+			if (in.inflow >> f & 1) {
 #pragma unroll
-			for (int ii = 0; ii < 6; ii++) {
-				T acc = T(0);
+				for (int ii = 0; ii < 6; ii++) {
+					T acc = T(0);
 #pragma unroll
-				for (int jj = 0; jj < 6; jj++)
-					if (!SPARSE || (smask(ii) >> jj & 1))
-						acc += tb.S[ii][jj] * tr[f][jj];
-				t[f2n(f, ii)] += acc * in.s[f];
+					for (int jj = 0; jj < 6; jj++)
+						if (!SPARSE || (smask(ii) >> jj & 1))
+							acc += tb.S[ii][jj] * x[f][jj];
+					t[f2n(f, ii)] += acc * in.s[f];
+				}
 			}
-		}
-#pragma unroll
-		for (int i = 0; i < 10; i++) {
-			T acc = T(0);
-#pragma unroll
-			for (int j = 0; j < 10; j++)
-				acc += tb.Minv[i][j] * t[j];
-			r[i] = in.fv[i] - in.coef * acc;
-		}
-	}
-	__pipeline_wait_prior(WAITG);
-	__syncthreads();
-	if (in.act) {
-		T y[10];
+		T mt[10], r[10];
+		lift_minv<T>(tb, t, mt);
+		load10<F, T>(sh.f + slot * 60 + c * 10, r);
 #pragma unroll
 		for (int i = 0; i < 10; i++)
-			y[i] = T(0);
-		const typename SG::vec *g = reinterpret_cast<const typename SG::vec *>(gsh + lane * SG::stride);
+			r[i] -= in.coef * mt[i];
+		block_product<T>(sh.G + slot * SweepCfg<T>::gstride, r, y);
+	}
+	if (FLOW) {
 #pragma unroll
-		for (int q = 0; q < 100 / SG::per_vec; q++) {
-			const typename SG::vec gv = g[q];
-			const T *ge = reinterpret_cast<const T *>(&gv);
+		for (int i = 0; i < 10; i++)
+			y[i] = written(y[i]);
+	}
+	__syncwarp(); // the item's rows are read: its y takes their place
+	if (in.act)
+		store10<T, T>(tr0 + c * 10, y);
+	__syncwarp();
+	if (in.act) {
+		T *yo = reinterpret_cast<T *>(p.y) + in.k * 60;
 #pragma unroll
-			for (int u = 0; u < SG::per_vec; u++) {
-				const int idx = q * SG::per_vec + u;
-				y[idx / 10] += ge[u] * r[idx % 10];
+		for (int i = 0; i < (YP + 5) / 6; i++)
+			if (c + 6 * i < YP)
+				*reinterpret_cast<float4 *>(yo + (c + 6 * i) * YV) =
+					*reinterpret_cast<const float4 *>(tr0 + (c + 6 * i) * YV);
+		if (ACC != 0) {
+			double2 *ya = reinterpret_cast<double2 *>(p.yacc + in.k * 60);
+#pragma unroll
+			for (int i = 0; i < 5; i++) {
+				const T *v = tr0 + 2 * (c + 6 * i);
+				ya[c + 6 * i] = ACC == 1 ? make_double2((double)v[0], (double)v[1])
+										 : make_double2(in.ya[ACC == 2 ? i : 0].x + (double)v[0],
+														in.ya[ACC == 2 ? i : 0].y + (double)v[1]);
 			}
 		}
-		store10<Y, T>(reinterpret_cast<Y *>(p.y) + k * 60 + c * 10, y);
-		if (ACC == 1) {
-			store10<double, T>(p.yacc + k * 60 + c * 10, y);
-		} else if (ACC == 2) {
-			double ya[10];
-#pragma unroll
-			for (int i = 0; i < 10; i++)
-				ya[i] = in.ya[i] + (double)y[i];
-			store10<double, double>(p.yacc + k * 60 + c * 10, ya);
-		}
 	}
-	if (FENCE)
-		__threadfence();
-	// gsh is reused by the CTA's next chunk
-	__syncthreads();
+	__syncwarp(); // the warp's shared memory is free for its next items
 }
 
-// One chunk, start to end.  `wait` is called by every thread between the
-// loads and the solve, with its item's inflow records nbk[4] (item index >= 0
-// for an upwind neighbour), its permutation records pmk[4] and whether the
-// thread holds an item.
-template <typename F, typename Y, typename T, int ACC, bool BD, bool SPARSE, bool L2, bool FENCE, typename Wait>
-__device__ __forceinline__ void sweep_chunk(const KinSweepParams &p, long long k0, long long item_end, T *gsh,
-											Wait wait, const int *list = nullptr)
+// the warp's share of the CTA's group [k0, k1): items k .. k + n - 1 (n <= 0: none)
+__device__ __forceinline__ int warp_items(long long k0, long long k1, long long &k)
 {
-	chunk_stage_G<T>(p, k0, chunk_nloc(k0, item_end), list, gsh);
-	ChunkIn<T, ACC> in;
-	chunk_load<F, T, ACC, BD>(p, k0, item_end, list, in);
-	wait(in.nbk, in.pmk, in.act);
-	chunk_solve<F, Y, T, ACC, BD, SPARSE, L2, FENCE, 0>(p, in, gsh);
+	k = k0 + kSwSlots * (threadIdx.x >> 5);
+	const long long n = k1 - k;
+	return n < kSwSlots ? (int)n : kSwSlots;
 }
 
+// One level per launch, with programmatic dependent launch: the next level's
+// CTAs stage their items (data no sweep level writes) while this level runs,
+// and wait (griddepcontrol.wait) only before they read the upwind rows.
 template <typename F, typename Y, typename T, int ACC, bool BD, bool SPARSE>
-__global__ void __launch_bounds__(kSwThreads) kin_sweep_kernel(KinSweepParams p)
+__global__ void __launch_bounds__(SweepCfg<T>::threads) kin_sweep_kernel(KinSweepParams p)
 {
-	__shared__ __align__(16) T gsh[kSwItems * SweepG<T>::stride];
-	// Programmatic dependent launch: the next level's CTAs may start now and
-	// run their prologue (everything before griddepcontrol.wait reads only
-	// data that no sweep level writes).
+	__shared__ SweepWarp<F, T> sh[SweepCfg<T>::warps];
 	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-	const long long k0 = (long long)p.item_begin + (long long)blockIdx.x * kSwItems;
-	// the upwind items of earlier levels are complete once the previous
-	// level's grid is
-	sweep_chunk<F, Y, T, ACC, BD, SPARSE, false, false>(
-		p, k0, p.item_end, gsh, [](const int *, const int *, bool) { asm volatile("griddepcontrol.wait;" ::: "memory"); });
+	long long k;
+	const int n = warp_items((long long)p.item_begin + (long long)blockIdx.x * SweepCfg<T>::items, p.item_end, k);
+	if (n <= 0)
+		return;
+	SweepLane<T, ACC> in;
+	warp_stage<F, T, ACC, BD>(p, k, n, nullptr, sh[threadIdx.x >> 5], in);
+	int nr[3];
+	T x[4][6];
+	inflow_rows(in, nr);
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+	warp_gather<F, T, ACC>(p, in, nr, sh[threadIdx.x >> 5], x);
+	warp_solve<F, T, ACC, SPARSE, false>(p, in, x, sh[threadIdx.x >> 5]);
 }
 
 // Grid-wide barrier of a cooperative launch (all CTAs co-resident).  *count
@@ -931,191 +1086,77 @@ static int launch_kin_kahn(const unsigned char *mask, const int *nb, const doubl
 }
 
 // All levels of one transport solve in one cooperative launch: the CTAs walk
-// the levels in order, 32 items per chunk, with a grid barrier between levels.
-// A CTA stages its first chunk of level l (G, records, right-hand side) before
-// it waits at the barrier that ends level l - 1.
+// the levels in order, one group of items at a time, with a grid barrier
+// between levels.  A CTA stages its first group of level l before it waits at
+// the barrier that ends level l - 1.
 template <typename F, typename Y, typename T, int ACC, bool BD, bool SPARSE>
-__global__ void __launch_bounds__(kSwThreads) kin_levels_kernel(KinSweepParams p, const int *__restrict__ level_off,
-																	int nlevels, unsigned *bar, int *err,
-																	long long spin_limit)
+__global__ void __launch_bounds__(SweepCfg<T>::threads)
+	kin_levels_kernel(KinSweepParams p, const int *__restrict__ level_off, int nlevels, unsigned *bar, int *err,
+					  long long spin_limit)
 {
-	__shared__ __align__(16) T gsh[kSwItems * SweepG<T>::stride];
+	__shared__ SweepWarp<F, T> sh[SweepCfg<T>::warps];
 	for (int l = 0; l < nlevels; l++) {
 		const long long b = level_off[l], e = level_off[l + 1];
-		const long long nch = (e - b + kSwItems - 1) / kSwItems;
+		const long long ng = (e - b + SweepCfg<T>::items - 1) / SweepCfg<T>::items;
 		bool pending = l > 0; // the barrier ending level l - 1 is still to pass
-		bool ok = true;
 		const unsigned target = (unsigned)l * gridDim.x;
-		for (long long ch = blockIdx.x; ch < nch; ch += gridDim.x) {
-			sweep_chunk<F, Y, T, ACC, BD, SPARSE, true, false>(p, b + ch * kSwItems, e, gsh, [&](const int *, const int *, bool) {
-				if (pending) {
-					ok = grid_barrier(bar, target, err, spin_limit);
-					pending = false;
-				}
-			});
-			if (!ok)
+		for (long long g = blockIdx.x; g < ng; g += gridDim.x) {
+			long long k;
+			const int n = warp_items(b + g * SweepCfg<T>::items, e, k);
+			SweepLane<T, ACC> in;
+			if (n > 0)
+				warp_stage<F, T, ACC, BD>(p, k, n, nullptr, sh[threadIdx.x >> 5], in);
+			if (pending && !grid_barrier(bar, target, err, spin_limit))
 				return;
+			pending = false;
+			if (n > 0) {
+				int nr[3];
+				T x[4][6];
+				inflow_rows(in, nr);
+				warp_gather<F, T, ACC>(p, in, nr, sh[threadIdx.x >> 5], x);
+				warp_solve<F, T, ACC, SPARSE, false>(p, in, x, sh[threadIdx.x >> 5]);
+			}
 		}
 		if (pending && !grid_barrier(bar, target, err, spin_limit))
 			return;
 	}
 }
 
-// Bounded wait for the readiness flags of an item's upwind neighbours
-// (need[f]): the flags are polled together with relaxed loads, and once all
-// are set one acquire fence orders the caller's later loads after the
-// producers' releases (the acquire pattern).  false when *err is set by
-// another CTA, or after spin_limit further polls (then *err is set here), so
-// a lost producer ends the launch instead of hanging it.  Only warp 0 of a CTA
-// waits; acquire loads one flag after another cost up to three L2 round trips
-// when the flags are already set.
-__device__ __forceinline__ bool wait_ready_all(const int *ready, const int nbk[4], const bool need[4], int *err,
-											   long long spin_limit)
-{
-	bool ok[4];
-#pragma unroll
-	for (int f = 0; f < 4; f++)
-		ok[f] = !need[f];
-	const volatile int *verr = err;
-	for (long long it = 0;; it++) {
-		int v[4];
-#pragma unroll
-		for (int f = 0; f < 4; f++) {
-			v[f] = 1;
-			if (!ok[f])
-				asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v[f]) : "l"(ready + nbk[f]) : "memory");
-		}
-		bool all = true;
-#pragma unroll
-		for (int f = 0; f < 4; f++) {
-			ok[f] = ok[f] || v[f] != 0;
-			all = all && ok[f];
-		}
-		if (all)
-			break;
-		if (*verr)
-			return false;
-		if (it >= spin_limit) {
-			atomicExch(err, 1);
-			return false;
-		}
-		if (it >= 32)
-			__nanosleep(32);
-	}
-	asm volatile("fence.acq_rel.gpu;" ::: "memory");
-	return true;
-}
-
-// The whole transport solve in one launch, driven by per-item readiness flags
-// instead of a barrier per level.  chunks[] lists the solve's 32-item chunks
-// in sweep order, never straddling a level, so every upwind item of a chunk
-// lies in an earlier chunk.  Each CTA takes the next chunk from an atomic
-// counter, stages it, waits (acquire, warp 0 only: a barrier then orders
-// the other warps' loads) for the flags of its own items' upwind neighbours,
-// solves, and publishes its items' flags (release).  A
-// chunk waits only on chunks taken earlier by CTAs already running, so the
-// solve progresses with any number of resident CTAs; the critical path is the
-// longest upwind chain, not the level count times a launch.  A CTA takes its
-// next ticket while it works on the current chunk (the smallest unfinished
-// chunk is still always being worked on).  Publication follows the barrier +
-// one release store pattern: the chunk's closing barrier orders every warp's
-// y stores before the release stores of the flags.  ready[] (one int per item)
-// and *queue are zero at launch.
+// The whole transport solve in one cooperative launch, driven by the rows
+// themselves (warp_gather_wait) instead of a barrier per level.  groups[] lists
+// items in sweep order in groups of one CTA's items, never straddling a level.
+// Without `group_off`, CTA b takes the groups b, b + gridDim.x, ... of the
+// whole sweep; with it, the groups group_off[b] .. group_off[b + 1] - 1 of its
+// own spatial part (their items in list[]; parts: equal ranges of elements
+// along a Morton curve of their centroids, all velocities of an element in one
+// part).  Each warp takes its five items of a group on its own.  All CTAs are
+// co-resident and walk their groups in sweep order, so the unfinished item of
+// lowest level always has its inputs and a warp at work on it: the solve
+// progresses, and its critical path is the longest upwind chain, not the level
+// count times a launch.
 template <typename F, typename Y, typename T, int ACC, bool BD, bool SPARSE>
-__global__ void __launch_bounds__(kSwThreads)
-	kin_flags_kernel(KinSweepParams p, const int2 *__restrict__ chunks, int nchunks, unsigned *queue, int *ready,
-					 int *err, long long spin_limit)
+__global__ void __launch_bounds__(SweepCfg<T>::threads)
+	kin_flow_kernel(KinSweepParams p, const int2 *__restrict__ groups, int ngroups, const int *__restrict__ list,
+					const int *__restrict__ group_off, int *err, long long spin_limit)
 {
-	__shared__ __align__(16) T gsh[kSwItems * SweepG<T>::stride];
-	__shared__ int s_chunk, s_fail;
-	int next = 0; // thread 0: the ticket taken ahead
-	if (threadIdx.x == 0)
-		next = (int)atomicAdd(queue, 1u);
-	for (;;) {
-		__syncthreads(); // the previous chunk's s_chunk / s_fail have been read
-		if (threadIdx.x == 0) {
-			s_chunk = next;
-			s_fail = 0;
-		}
-		__syncthreads();
-		const int c = s_chunk;
-		if (c >= nchunks)
-			return;
-		if (threadIdx.x == 0)
-			next = (int)atomicAdd(queue, 1u);
-		const int2 ck = chunks[c];
-		sweep_chunk<F, Y, T, ACC, BD, SPARSE, true, false>(
-			p, ck.x, ck.y, gsh, [&](const int *nbk, const int *, bool act) {
-				// warp 0 waits for the chunk; the barrier orders the other
-				// warps' trace loads after its acquires
-				if (threadIdx.x < 32 && act) {
-					bool need[4];
-#pragma unroll
-					for (int f = 0; f < 4; f++)
-						need[f] = nbk[f] >= 0;
-					if (!wait_ready_all(ready, nbk, need, err, spin_limit))
-						s_fail = 1;
-				}
-				__syncthreads();
-			});
-		// sweep_chunk ended with a barrier after every thread's y stores
-		if (s_fail)
+	__shared__ SweepWarp<F, T> sh[SweepCfg<T>::warps];
+	const int g0 = group_off ? group_off[blockIdx.x] : blockIdx.x;
+	const int g1 = group_off ? group_off[blockIdx.x + 1] : ngroups;
+	const int dg = group_off ? 1 : gridDim.x;
+	for (int g = g0; g < g1; g += dg) {
+		const int2 gr = groups[g];
+		long long k;
+		const int n = warp_items(gr.x, gr.y, k);
+		if (n <= 0)
+			continue;
+		SweepLane<T, ACC> in;
+		warp_stage<F, T, ACC, BD>(p, k, n, list, sh[threadIdx.x >> 5], in);
+		int nr[3];
+		T x[4][6];
+		inflow_rows(in, nr);
+		if (!warp_gather_wait<F, T, ACC>(p, in, nr, sh[threadIdx.x >> 5], x, err, spin_limit))
 			return; // *err is set; the state of this solve is invalid
-		if (threadIdx.x < ck.y - ck.x)
-			asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(ready + ck.x + threadIdx.x), "r"(1)
-						 : "memory");
-	}
-}
-
-// The whole transport solve in one cooperative launch, each CTA sweeping one
-// spatial part of the mesh.  Elements are split into compact parts (equal
-// ranges along a Morton curve of their centroids; all velocities of an element
-// in one part), and part b's items are listed in sweep order in plist[], cut
-// into chunks (pchunks[c] = first list position, count) that never straddle a
-// level.  CTA b walks its chunks in order, so an upwind item in its own part
-// was solved by an earlier chunk of the same CTA (the chunk's closing barrier
-// orders it); only an upwind item of another part, marked by bit 28 of the
-// face's permutation record, is waited for through its readiness flag
-// (acquire), and every chunk publishes its items' flags (release).  All CTAs
-// are co-resident (cooperative launch), and the unfinished item of lowest
-// level always belongs to a chunk whose part is working on it, so the solve
-// progresses; the waits are bounded as in the flag-driven sweep.  Inside a
-// part a dependent step costs one chunk (a barrier, traces through L2, the
-// block solve) instead of one launch per level.
-constexpr int kPartExternal = 1 << 28;
-template <typename F, typename Y, typename T, int ACC, bool BD, bool SPARSE>
-__global__ void __launch_bounds__(kSwThreads)
-	kin_parts_kernel(KinSweepParams p, const int *__restrict__ plist, const int2 *__restrict__ pchunks,
-					 const int *__restrict__ part_chunk_off, int *ready, int *err, long long spin_limit)
-{
-	__shared__ __align__(16) T gsh[kSwItems * SweepG<T>::stride];
-	__shared__ int s_fail;
-	if (threadIdx.x == 0)
-		s_fail = 0;
-	__syncthreads();
-	const int c_end = part_chunk_off[blockIdx.x + 1];
-	for (int c = part_chunk_off[blockIdx.x]; c < c_end; c++) {
-		const int2 ck = pchunks[c];
-		sweep_chunk<F, Y, T, ACC, BD, SPARSE, true, false>(
-			p, ck.x, ck.x + ck.y, gsh,
-			[&](const int *nbk, const int *pmk, bool act) {
-				if (threadIdx.x < 32 && act) {
-					bool need[4];
-#pragma unroll
-					for (int f = 0; f < 4; f++)
-						need[f] = nbk[f] >= 0 && (pmk[f] & kPartExternal);
-					if (!wait_ready_all(ready, nbk, need, err, spin_limit))
-						s_fail = 1;
-				}
-				__syncthreads();
-			},
-			plist);
-		// sweep_chunk ended with a barrier after every thread's y stores
-		if (s_fail)
-			return; // *err is set; the state of this solve is invalid
-		if (threadIdx.x < ck.y)
-			asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(ready + plist[ck.x + threadIdx.x]), "r"(1)
-						 : "memory");
+		warp_solve<F, T, ACC, SPARSE, true>(p, in, x, sh[threadIdx.x >> 5]);
 	}
 }
 
@@ -1166,30 +1207,11 @@ __global__ void kin_part_of_item_kernel(const int *__restrict__ items, const int
 	part_key[k] = part_of_elem[items[k] / nv];
 	iota[k] = (int)k;
 }
-// bit 28 of rpm[k].f: the upwind item across face f belongs to another part
-__global__ void kin_mark_external_kernel(const int4 *__restrict__ rnb, const int *__restrict__ part_of_item,
-										 long long nitems, int4 *__restrict__ rpm)
-{
-	const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-	if (k >= nitems)
-		return;
-	const int4 nb = rnb[k];
-	int4 pm = rpm[k];
-	const int me = part_of_item[k];
-	const int n[4] = {nb.x, nb.y, nb.z, nb.w};
-	int m[4] = {pm.x & ~kPartExternal, pm.y & ~kPartExternal, pm.z & ~kPartExternal, pm.w & ~kPartExternal};
-	for (int f = 0; f < 4; f++)
-		if (n[f] >= 0 && part_of_item[n[f]] != me)
-			m[f] |= kPartExternal;
-	rpm[k] = make_int4(m[0], m[1], m[2], m[3]);
-}
-
-// Spatial parts of the item list (kin_parts_kernel): nparts compact element
+// Spatial parts of the item list (kin_flow_kernel): nparts compact element
 // parts; on return plist (device, [nitems]: items of part 0 in sweep order,
-// then part 1, ...), pkey_host (host, [nitems]: the part of plist[i]) and the
-// external-dependency bits of rpm are set.
+// then part 1, ...) and pkey_host (host, [nitems]: the part of plist[i]) are set.
 int kin_build_parts(const int *e2q, const double *node, long long ne, const double lo[3], const double hi[3],
-					const int *items, long long nitems, int nv, int nparts, const int4 *rnb, int4 *rpm, int *plist,
+					const int *items, long long nitems, int nv, int nparts, int *plist,
 					std::vector<int> &plist_host, std::vector<int> &pkey_host, cudaStream_t s)
 {
 	unsigned *code = nullptr, *code_s = nullptr;
@@ -1239,8 +1261,6 @@ int kin_build_parts(const int *e2q, const double *node, long long ne, const doub
 	GDN_PARTS_TRY(cudaGetLastError());
 	kin_part_of_item_kernel<<<gi, 256, 0, s>>>(items, pe, nitems, nv, pkey, iota);
 	GDN_PARTS_TRY(cudaGetLastError());
-	kin_mark_external_kernel<<<gi, 256, 0, s>>>(rnb, pkey, nitems, rpm);
-	GDN_PARTS_TRY(cudaGetLastError());
 	int bits = 1;
 	while ((1 << bits) <= nparts)
 		bits++;
@@ -1257,78 +1277,14 @@ int kin_build_parts(const int *e2q, const double *node, long long ne, const doub
 }
 
 template <typename F, typename Y, typename T>
-int launch_kin_parts(const KinSweepParams &p, const int *plist, const int2 *pchunks, const int *part_chunk_off,
-					 int nparts, int *ready, long long nitems, int *err, long long spin, int acc, int bdata,
-					 int sparse, cudaStream_t s)
-{
-	if (nparts <= 0)
-		return GDN_CUDA_OK;
-	GDN_CUDA_TRY(cudaMemsetAsync(ready, 0, (size_t)nitems * sizeof(int), s));
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3((unsigned)nparts);
-	cfg.blockDim = dim3(kSwThreads);
-	cfg.dynamicSmemBytes = 0;
-	cfg.stream = s;
-	cudaLaunchAttribute attr[1];
-	attr[0].id = cudaLaunchAttributeCooperative;
-	attr[0].val.cooperative = 1;
-	cfg.attrs = attr;
-	cfg.numAttrs = 1;
-#define GDN_PARTS(A, B, SP)                                                                                           \
-	GDN_CUDA_TRY(cudaLaunchKernelEx(&cfg, kin_parts_kernel<F, Y, T, A, B, SP>, p, plist, pchunks, part_chunk_off,    \
-									ready, err, spin))
-	if (acc == 0 && bdata) {
-		if (sparse)
-			GDN_PARTS(0, true, true);
-		else
-			GDN_PARTS(0, true, false);
-	} else if (acc == 1 && bdata) {
-		if (sparse)
-			GDN_PARTS(1, true, true);
-		else
-			GDN_PARTS(1, true, false);
-	} else if (acc == 2 && !bdata) {
-		if (sparse)
-			GDN_PARTS(2, false, true);
-		else
-			GDN_PARTS(2, false, false);
-	} else {
-		return gdn_set_error(GDN_CUDA_ERR_INVALID, "kinetic sweep: unsupported accumulate / boundary mode");
-	}
-#undef GDN_PARTS
-	GDN_CUDA_TRY(cudaGetLastError());
-	return GDN_CUDA_OK;
-}
-
-// CTAs of the spatial-parts sweep that fit on the device at once
-template <typename F, typename Y, typename T>
-int kin_parts_grid(int device, int acc, int sparse, int *grid)
-{
-	int nsm = 0, per = 0;
-	GDN_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
-	const void *fn;
-	if (sparse)
-		fn = acc == 0   ? (const void *)kin_parts_kernel<F, Y, T, 0, true, true>
-			 : acc == 1 ? (const void *)kin_parts_kernel<F, Y, T, 1, true, true>
-						: (const void *)kin_parts_kernel<F, Y, T, 2, false, true>;
-	else
-		fn = acc == 0   ? (const void *)kin_parts_kernel<F, Y, T, 0, true, false>
-			 : acc == 1 ? (const void *)kin_parts_kernel<F, Y, T, 1, true, false>
-						: (const void *)kin_parts_kernel<F, Y, T, 2, false, false>;
-	GDN_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kSwThreads, 0));
-	*grid = nsm * (per > 0 ? per : 1);
-	return GDN_CUDA_OK;
-}
-
-template <typename F, typename Y, typename T>
 int launch_kin_sweep(const KinSweepParams &p, int acc, int bdata, int sparse, cudaStream_t s)
 {
 	const long long n = (long long)p.item_end - p.item_begin;
 	if (n <= 0)
 		return GDN_CUDA_OK;
 	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3((unsigned)((n + kSwItems - 1) / kSwItems));
-	cfg.blockDim = dim3(kSwThreads);
+	cfg.gridDim = dim3((unsigned)((n + SweepCfg<T>::items - 1) / SweepCfg<T>::items));
+	cfg.blockDim = dim3(SweepCfg<T>::threads);
 	cfg.dynamicSmemBytes = 0;
 	cfg.stream = s;
 	cudaLaunchAttribute attr[1];
@@ -1365,7 +1321,7 @@ int launch_kin_levels(const KinSweepParams &p, const int *level_off, int nlevels
 {
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3((unsigned)grid);
-	cfg.blockDim = dim3(kSwThreads);
+	cfg.blockDim = dim3(SweepCfg<T>::threads);
 	cfg.dynamicSmemBytes = 0;
 	cfg.stream = s;
 	cudaLaunchAttribute attr[1];
@@ -1400,58 +1356,69 @@ int launch_kin_levels(const KinSweepParams &p, const int *level_off, int nlevels
 }
 
 template <typename F, typename Y, typename T>
-int launch_kin_flags(const KinSweepParams &p, const int2 *chunks, int nchunks, int grid, unsigned *queue, int *ready,
-					 long long nitems, int *err, long long spin, int acc, int bdata, int sparse, cudaStream_t s)
+int launch_kin_flow(const KinSweepParams &p, const int2 *groups, int ngroups, const int *list, const int *group_off,
+					int grid, long long nitems, int *err, long long spin, int acc, int bdata, int sparse,
+					cudaStream_t s)
 {
-	if (nchunks <= 0)
+	if (ngroups <= 0)
 		return GDN_CUDA_OK;
-	GDN_CUDA_TRY(cudaMemsetAsync(ready, 0, (size_t)nitems * sizeof(int), s));
-	GDN_CUDA_TRY(cudaMemsetAsync(queue, 0, sizeof(unsigned), s));
-	const unsigned g = (unsigned)(grid < nchunks ? grid : nchunks);
-#define GDN_FLAGS(A, B, SP)                                                                                           \
-	kin_flags_kernel<F, Y, T, A, B, SP><<<g, kSwThreads, 0, s>>>(p, chunks, nchunks, queue, ready, err, spin)
+	// every row unwritten (clearing it in the relaxation, which reads y anyway,
+	// measured slower: 3.79 against 3.62 ms per 64^3 FP32 step)
+	GDN_CUDA_TRY(cudaMemsetAsync(p.y, 0xff, (size_t)nitems * 60 * sizeof(Y), s));
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3((unsigned)grid);
+	cfg.blockDim = dim3(SweepCfg<T>::threads);
+	cfg.stream = s;
+	cudaLaunchAttribute attr[1];
+	attr[0].id = cudaLaunchAttributeCooperative;
+	attr[0].val.cooperative = 1;
+	cfg.attrs = attr;
+	cfg.numAttrs = 1;
+#define GDN_FLOW(A, B, SP)                                                                                            \
+	GDN_CUDA_TRY(cudaLaunchKernelEx(&cfg, kin_flow_kernel<F, Y, T, A, B, SP>, p, groups, ngroups, list, group_off,   \
+									err, spin))
 	if (acc == 0 && bdata) {
 		if (sparse)
-			GDN_FLAGS(0, true, true);
+			GDN_FLOW(0, true, true);
 		else
-			GDN_FLAGS(0, true, false);
+			GDN_FLOW(0, true, false);
 	} else if (acc == 1 && bdata) {
 		if (sparse)
-			GDN_FLAGS(1, true, true);
+			GDN_FLOW(1, true, true);
 		else
-			GDN_FLAGS(1, true, false);
+			GDN_FLOW(1, true, false);
 	} else if (acc == 2 && !bdata) {
 		if (sparse)
-			GDN_FLAGS(2, false, true);
+			GDN_FLOW(2, false, true);
 		else
-			GDN_FLAGS(2, false, false);
+			GDN_FLOW(2, false, false);
 	} else {
 		return gdn_set_error(GDN_CUDA_ERR_INVALID, "kinetic sweep: unsupported accumulate / boundary mode");
 	}
-#undef GDN_FLAGS
+#undef GDN_FLOW
 	GDN_CUDA_TRY(cudaGetLastError());
 	return GDN_CUDA_OK;
 }
 
-// CTAs of the flag-driven sweep that fit on the device at once
+// CTAs of the row-driven sweep that fit on the device at once
 template <typename F, typename Y, typename T>
-int kin_flags_grid(int device, int acc, int sparse, int *grid)
+int kin_flow_grid(int device, int acc, int sparse, int *grid)
 {
 	int nsm = 0, per = 0;
 	GDN_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
 	const void *fn;
 	if (sparse)
-		fn = acc == 0   ? (const void *)kin_flags_kernel<F, Y, T, 0, true, true>
-			 : acc == 1 ? (const void *)kin_flags_kernel<F, Y, T, 1, true, true>
-						: (const void *)kin_flags_kernel<F, Y, T, 2, false, true>;
+		fn = acc == 0   ? (const void *)kin_flow_kernel<F, Y, T, 0, true, true>
+			 : acc == 1 ? (const void *)kin_flow_kernel<F, Y, T, 1, true, true>
+						: (const void *)kin_flow_kernel<F, Y, T, 2, false, true>;
 	else
-		fn = acc == 0   ? (const void *)kin_flags_kernel<F, Y, T, 0, true, false>
-			 : acc == 1 ? (const void *)kin_flags_kernel<F, Y, T, 1, true, false>
-						: (const void *)kin_flags_kernel<F, Y, T, 2, false, false>;
-	GDN_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kSwThreads, 0));
-	// at most 4 CTAs per SM: the chunks in flight then poll and publish least
-	// against each other (64^3 FP32 ms per step for 2 to 6 CTAs per SM: 5.20,
-	// 4.56, 4.35, 4.46, 4.54)
+		fn = acc == 0   ? (const void *)kin_flow_kernel<F, Y, T, 0, true, false>
+			 : acc == 1 ? (const void *)kin_flow_kernel<F, Y, T, 1, true, false>
+						: (const void *)kin_flow_kernel<F, Y, T, 2, false, false>;
+	GDN_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, SweepCfg<T>::threads, 0));
+	// at most 4 CTAs per SM: more warps in flight only poll (ms per step for 2, 3,
+	// 4 CTAs per SM and all that fit: 64^3 FP32 4.46, 3.93, 3.79, 3.80; 40^3 FP64
+	// 2.00, 1.93, 1.94, 1.94; 17^3 FP64 0.439, 0.443, 0.445, 0.450)
 	const int cap = 4;
 	*grid = nsm * (per > cap ? cap : (per > 0 ? per : 1));
 	return GDN_CUDA_OK;
@@ -1472,10 +1439,10 @@ int kin_levels_grid(int device, int acc, int sparse, int *grid)
 		fn = acc == 0   ? (const void *)kin_levels_kernel<F, Y, T, 0, true, false>
 			 : acc == 1 ? (const void *)kin_levels_kernel<F, Y, T, 1, true, false>
 						: (const void *)kin_levels_kernel<F, Y, T, 2, false, false>;
-	GDN_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kSwThreads, 0));
-	// at most 3 CTAs per SM, about one per 32-item chunk of a 64^3 level: fewer
-	// arrivals per grid barrier (64^3 FP32 ms per step for 2 / 3 / 4 CTAs per
-	// SM: 6.04, 5.81, 6.75)
+	GDN_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, SweepCfg<T>::threads, 0));
+	// at most 3 CTAs per SM, about one per group of a 64^3 level: fewer arrivals
+	// per grid barrier (ms per step for 1, 2, 3, 4 CTAs per SM: 64^3 FP32 8.31,
+	// 6.41, 5.98, 5.89; 40^3 FP64 3.69, 3.06, 3.07, 3.10)
 	*grid = nsm * (per > 3 ? 3 : per);
 	return GDN_CUDA_OK;
 }
@@ -1484,12 +1451,9 @@ int kin_levels_grid(int device, int acc, int sparse, int *grid)
 	template int launch_kin_levels<F, Y, T>(const KinSweepParams &, const int *, int, int, unsigned *, int *,         \
 											long long, int, int, int, cudaStream_t);                                     \
 	template int kin_levels_grid<F, Y, T>(int, int, int, int *);                                                      \
-	template int launch_kin_flags<F, Y, T>(const KinSweepParams &, const int2 *, int, int, unsigned *, int *,         \
-										   long long, int *, long long, int, int, int, cudaStream_t);                    \
-	template int kin_flags_grid<F, Y, T>(int, int, int, int *);                                                       \
-	template int launch_kin_parts<F, Y, T>(const KinSweepParams &, const int *, const int2 *, const int *, int,       \
-										   int *, long long, int *, long long, int, int, int, cudaStream_t);             \
-	template int kin_parts_grid<F, Y, T>(int, int, int, int *);
+	template int launch_kin_flow<F, Y, T>(const KinSweepParams &, const int2 *, int, const int *, const int *, int,   \
+										  long long, int *, long long, int, int, int, cudaStream_t);                     \
+	template int kin_flow_grid<F, Y, T>(int, int, int, int *);
 GDN_LEVELS_INST(double, double, double)
 GDN_LEVELS_INST(float, float, float)
 GDN_LEVELS_INST(__nv_bfloat16, float, float)
@@ -1507,11 +1471,12 @@ template int launch_kin_sweep<double, float, float>(const KinSweepParams &, int,
 // with V_ij = -(u . D_ij), u_k = v . codtau[:, k], tr the upwind neighbour's
 // y or the boundary f_eq.  This is f - b - M1 y with M1 as the blocks kernel
 // builds it, from the FP64 u, theta dt / det and v.vn it records per item.
+constexpr int kResThreads = 192;
 template <bool SPARSE>
-__global__ void __launch_bounds__(kSwThreads) kin_residual_kernel(KinResidualParams p)
+__global__ void __launch_bounds__(kResThreads) kin_residual_kernel(KinResidualParams p)
 {
 	const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
-	const long long k = (long long)blockIdx.x * kSwItems + lane;
+	const long long k = (long long)blockIdx.x * 32 + lane;
 	if (k >= p.nitems)
 		return;
 	const Tables<double> &tb = c_tab_d;
@@ -1591,11 +1556,11 @@ int launch_kin_residual(const KinResidualParams &p, int sparse, cudaStream_t s)
 {
 	if (p.nitems <= 0)
 		return GDN_CUDA_OK;
-	const unsigned grid = (unsigned)((p.nitems + kSwItems - 1) / kSwItems);
+	const unsigned grid = (unsigned)((p.nitems + 31) / 32);
 	if (sparse)
-		kin_residual_kernel<true><<<grid, kSwThreads, 0, s>>>(p);
+		kin_residual_kernel<true><<<grid, kResThreads, 0, s>>>(p);
 	else
-		kin_residual_kernel<false><<<grid, kSwThreads, 0, s>>>(p);
+		kin_residual_kernel<false><<<grid, kResThreads, 0, s>>>(p);
 	GDN_CUDA_TRY(cudaGetLastError());
 	return GDN_CUDA_OK;
 }

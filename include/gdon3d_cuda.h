@@ -134,12 +134,11 @@ typedef struct gdn_cuda_config {
 	int device; /* CUDA device ordinal */
 	int kin_sweep; /* kinetic transport solve: 1 = a launch per sweep level,
 	                  2 = one cooperative launch walking all levels with a
-	                  grid barrier between them, 3 = one launch driven by
-	                  per-item readiness flags (CTAs take 32-item chunks in
-	                  sweep order and wait only for their upwind neighbours),
-	                  4 = one cooperative launch in which each CTA sweeps one
-	                  compact spatial part of the mesh in sweep order and
-	                  waits only for upwind items of other parts,
+	                  grid barrier between them, 3 = one cooperative launch
+	                  driven by the solution itself (warps take five items in
+	                  sweep order and wait until their upwind neighbours'
+	                  values are written), 4 = the same with each CTA sweeping
+	                  one compact spatial part of the mesh in sweep order,
 	                  0 = the fastest of the four, timed at attach and cached
 	                  per (precision, size) */
 } gdn_cuda_config;
@@ -322,7 +321,7 @@ int gdn_cuda_num_instances(gdn_cuda_handle *h, int *ninst);
 int gdn_cuda_kin_sweep_mode(gdn_cuda_handle *h, int *mode);
 /* Test and diagnostics hook, no counterpart in the reference: the number of
  * polls after which a bounded device-side wait (the cooperative sweep's grid
- * barrier, the flag-driven and spatial-parts sweeps' readiness waits) gives up, sets the
+ * barrier, the row waits of modes 3 and 4) gives up, sets the
  * handle's error flag and lets its launch end; the next call that reads the
  * state back (get_state, solve, step_host, error_l2, save_xdmf) then returns
  * GDN_CUDA_ERR_TIMEOUT and the state is invalid until it is set again.
