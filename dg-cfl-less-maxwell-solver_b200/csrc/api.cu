@@ -1922,7 +1922,7 @@ extern "C" int gdn_cuda_rk3_variant(gdn_cuda_handle *h, int *variant, int *min_c
 	const bool rk = h->scheme == GDN_CUDA_SCHEME_RK3;
 	*variant = rk ? h->rk3_variant + 1 : 0;
 	if (min_ctas_per_sm)
-		*min_ctas_per_sm = rk ? rk3_min_blocks(h->precision == GDN_CUDA_FP64, h->rk3_variant) : 0;
+		*min_ctas_per_sm = rk ? rk3_min_blocks(h->precision == GDN_CUDA_FP64, h->rk3_fact, h->rk3_variant) : 0;
 	return GDN_CUDA_OK;
 }
 

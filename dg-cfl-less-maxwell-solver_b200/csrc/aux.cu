@@ -94,7 +94,7 @@ __global__ void init_rk3_kernel(const int *__restrict__ e2q, const double *__res
 	node_xyz(e2q, node, e, i, x);
 	exact_w(d, x, 0.0, we);
 	for (int c = 0; c < 6; c++)
-		Store<S>::store(w + rk3_tix(e0 + e, i * 6 + c), we[c]);
+		Store<S>::store(w + rk3_tix<S>(e0 + e, i * 6 + c), we[c]);
 }
 
 template <typename S>
@@ -182,7 +182,7 @@ __global__ void boundary_dofs_kernel(const double *__restrict__ bxyz, long long 
 }
 
 // RK3 boundary traces at a stage time, in the stage kernels' precision:
-// out[(bf*6 + jj)*6 + c] = w_exact(x_{bf,jj}, t)_c  (dg_update_boundary,
+// out[(bf*6 + jj)*6 + rk3_btrace_off(c)] = w_exact(x_{bf,jj}, t)_c  (dg_update_boundary,
 // dg.c:101-104, evaluated once per stage instead of inside the flux loop),
 // with the data, time and time step of the face's instance.  The stage time
 // t + C_i dt is formed from the device copy of t with the host's rounding (no
@@ -199,7 +199,7 @@ __global__ void boundary_trace_kernel(const double *__restrict__ bxyz, long long
 	double x[3] = {bxyz[3 * u], bxyz[3 * u + 1], bxyz[3 * u + 2]}, we[6];
 	exact_w(b.data[inst], x, t, we);
 	for (int c = 0; c < 6; c++)
-		out[u * 6 + c] = (T)we[c];
+		out[u * 6 + rk3_btrace_off<T>(c)] = (T)we[c];
 }
 
 template <typename T>
@@ -335,7 +335,7 @@ __global__ void error_partial_kernel(const S *__restrict__ state, int kinetic, l
 		exact_w(d, x, t, we);
 		if (!kinetic) {
 			for (int c = 0; c < 6; c++)
-				wl[c] = (double)Store<S>::load(state + rk3_tix(e0 + e, i * 6 + c));
+				wl[c] = (double)Store<S>::load(state + rk3_tix<S>(e0 + e, i * 6 + c));
 		} else {
 			for (int c = 0; c < 6; c++) {
 				double s = 0.0;
@@ -440,7 +440,7 @@ __global__ void io_values_kernel(const S *__restrict__ st, int kinetic, int nv, 
 	const int i = u % 10;
 	if (!kinetic) {
 		for (int c = 0; c < 6; c++)
-			out[c * nq + in] = (double)Store<S>::load(st + rk3_tix(e, i * 6 + c));
+			out[c * nq + in] = (double)Store<S>::load(st + rk3_tix<S>(e, i * 6 + c));
 	} else {
 		// component im = iw * nv + iv of the reference's kinetic wn
 		for (int v = 0; v < nv; v++) {

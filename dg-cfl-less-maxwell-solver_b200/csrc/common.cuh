@@ -80,10 +80,32 @@ __device__ __forceinline__ const Tables<float> &tab<float>()
 }
 
 // RK3 device layout: tiles of 32 elements, value-major inside a tile; value k
-// (= node * 6 + field) of element e.
+// (= node * 6 + field) of element e.  FP64: one field per row of 32 elements.
+// FP32: rows of 32 (E_c, H_c) pairs, so that a lane moves and computes both
+// halves of a component at once (packed FP32x2).
+template <typename T>
 __host__ __device__ __forceinline__ long long rk3_tix(long long e, int k)
 {
+	if (sizeof(T) == 4)
+		return ((e >> 5) * 30 + k / 6 * 3 + k % 3) * 64 + (e & 31) * 2 + k % 6 / 3;
 	return ((e >> 5) * 60 + k) * 32 + (e & 31);
+}
+// the same within a tile, for a lane whose element starts at rk3_lane: field c
+// of a node, and value c of a boundary trace
+template <typename T>
+__host__ __device__ __forceinline__ int rk3_lane(int lane)
+{
+	return sizeof(T) == 4 ? 2 * lane : lane;
+}
+template <typename T>
+__host__ __device__ __forceinline__ int rk3_off(int node, int c)
+{
+	return sizeof(T) == 4 ? (node * 3 + c % 3) * 64 + c / 3 : (node * 6 + c) * 32;
+}
+template <typename T>
+__host__ __device__ __forceinline__ int rk3_btrace_off(int c)
+{
+	return sizeof(T) == 4 ? c % 3 * 2 + c / 3 : c;
 }
 
 // Analytic data (boundary values, initial data, error norm), FP64.

@@ -50,13 +50,14 @@ void rk3_sym_coeffs(const gdn_cuda_tables *t, double q4_sym[6], double minv_sym[
 bool rk3_tables_standard_faces(const gdn_cuda_tables *t);
 
 // variant 0 / 1: the stage kernel compiled for fewer / more resident CTAs per
-// SM (rk3_min_blocks), i.e. more / fewer registers per thread
+// SM (rk3_min_blocks), i.e. more / fewer registers per thread; FP32 with the P2
+// tables: rk3_elem_kernel (a thread per element), else rk3_stage_kernel
 template <typename T>
 int launch_rk3_stage(const Rk3Params<T> &p, int variant, cudaStream_t s);
 template <typename T>
 int prepare_rk3();
 
-int rk3_min_blocks(int precision_fp64, int variant);
+int rk3_min_blocks(int precision_fp64, int fact, int variant);
 // reference layout [e][node][field] (FP64, elements 0..ne-1) <-> tiled layout
 // at elements e0 .. e0 + ne - 1
 template <typename T>

@@ -20,7 +20,7 @@
 // before the stage.
 //
 // Device layout: the state, k2 and the geometry are stored in tiles of 32
-// elements, value-major inside a tile (rk3_tix): value k of element e at
+// elements, value-major inside a tile (rk3_tix): FP64 value k of element e at
 // ((e / 32) * 60 + k) * 32 + e % 32.  A CTA owns one tile with 6 warps, lane =
 // element, so every per-element access of a warp is one coalesced 128-byte
 // (FP32) row:
@@ -37,6 +37,7 @@
 //   -- the one barrier --
 //   3  warp c: R_c = curl part + sum_faces S F_c, lift by Minv, RK update with
 //      k2 (loaded before the barrier), coalesced stores.
+// FP32 with the P2 tables runs rk3_elem_kernel instead: a thread per element.
 #include <cmath>
 
 #include "common.cuh"
@@ -247,14 +248,16 @@ struct Rk3Smem {
 	static constexpr int bytes_fact = 144 * P * (int)sizeof(T);
 };
 
-// The two autotuned CTA-per-tile variants: register cap (minimum resident
-// CTAs per SM) and how the neighbour traces are prefetched (rk3_tile).
+// The two autotuned variants of rk3_stage_kernel: register cap (minimum
+// resident CTAs per SM) and how the neighbour traces are prefetched (rk3_tile).
+// FP32 runs it only for tables without the P2 symmetry (rk3_elem_kernel
+// otherwise).
 template <typename T>
 struct Rk3Variants;
 template <>
 struct Rk3Variants<float> {
 	static constexpr int lo = 4, hi = 5;
-	static constexpr int pf_lo = 2, pf_hi = 2; // PF_ASYNC: 77 / 64 registers
+	static constexpr int pf_lo = 0, pf_hi = 0; // PF_NONE: the pair layout has no constant field stride
 };
 template <>
 struct Rk3Variants<double> {
@@ -290,38 +293,6 @@ __device__ __forceinline__ void upwind_flux_h(const T wL[6], const T wR[6], cons
 	F[5] = (h[0] * sE[1] - h[1] * sE[0]) + r2 * (n[2] * nH - nn * dH[2]);
 }
 
-// FP32: the same flux with the (E_k, H_k) component pairs in packed FP32x2
-// arithmetic: d = wR - wL and t_k = n_k (n . d) - |n|^2 d_k per pair, the
-// cross products from the swapped sums (sH_k, sE_k):
-// (F_E, F_H)_k = (1, -1) (h_{k+2} sw_{k+1} - h_{k+1} sw_{k+2}) + r2 t_k.
-template <>
-__device__ __forceinline__ void upwind_flux_h<float>(const float wL[6], const float wR[6], const float n[3],
-													 float F[6])
-{
-	const float nn = n[0] * n[0] + n[1] * n[1] + n[2] * n[2];
-	const float r2 = 0.5f * inv_norm_eps(nn);
-	const float2 m1 = make_float2(-1.f, -1.f);
-	float2 d[3], sw[3];
-#pragma unroll
-	for (int k = 0; k < 3; k++) {
-		d[k] = __ffma2_rn(make_float2(wL[k], wL[3 + k]), m1, make_float2(wR[k], wR[3 + k]));
-		sw[k] = __fadd2_rn(make_float2(wR[3 + k], wR[k]), make_float2(wL[3 + k], wL[k]));
-	}
-	const float2 nd = __ffma2_rn(make_float2(n[2], n[2]), d[2],
-								 __ffma2_rn(make_float2(n[1], n[1]), d[1], __fmul2_rn(make_float2(n[0], n[0]), d[0])));
-	const float2 mnn = make_float2(-nn, -nn), rr = make_float2(r2, r2), pm = make_float2(1.f, -1.f);
-#pragma unroll
-	for (int k = 0; k < 3; k++) {
-		const int k1 = (k + 1) % 3, k2 = (k + 2) % 3;
-		const float h1 = 0.5f * n[k1], h2 = 0.5f * n[k2];
-		const float2 t = __ffma2_rn(mnn, d[k], __fmul2_rn(make_float2(n[k], n[k]), nd));
-		const float2 u = __ffma2_rn(make_float2(-h1, -h1), sw[k2], __fmul2_rn(make_float2(h2, h2), sw[k1]));
-		const float2 Fk = __ffma2_rn(u, pm, __fmul2_rn(rr, t));
-		F[k] = Fk.x;
-		F[3 + k] = Fk.y;
-	}
-}
-
 // One tile of 32 elements, phases 1-3 (all threads of the CTA call it: it
 // holds the barrier between phases 2 and 3).  Wt[k * 32] is value k of this
 // lane's element (global memory or a shared-memory copy of the tile), Gt[q *
@@ -349,15 +320,15 @@ __device__ __forceinline__ void rk3_tile(const Rk3Params<T> &p, long long tile, 
 		const int jj = warp;
 		if (nbv >= 0) {
 			const int qn = (pmk[f] >> (4 * jj)) & 15;
-			const T *g = p.w_in + rk3_tix(nbv, qn * 6);
+			const T *g = p.w_in + rk3_tix<T>(nbv, qn * 6);
 #pragma unroll
 			for (int c = 0; c < 6; c++)
-				out[c] = __ldg(g + c * 32);
+				out[c] = __ldg(g + rk3_off<T>(0, c));
 		} else {
 			const T *g = p.btrace + ((long long)(-nbv - 1) * 6 + jj) * 6;
 #pragma unroll
 			for (int c = 0; c < 6; c++)
-				out[c] = __ldg(g + c);
+				out[c] = __ldg(g + rk3_btrace_off<T>(c));
 		}
 	};
 	// Prefetched at the start so that the volume phase hides their latency:
@@ -384,7 +355,7 @@ __device__ __forceinline__ void rk3_tile(const Rk3Params<T> &p, long long tile, 
 				if (nbv >= 0) {
 					const unsigned qn = ((unsigned)pmk[f] >> (4 * warp)) & 15u;
 					const T *g = p.idx32 ? p.w_in + (((unsigned)nbv >> 5) * 1920u + qn * 192u + ((unsigned)nbv & 31u))
-										 : p.w_in + rk3_tix(nbv, (int)qn * 6);
+										 : p.w_in + rk3_tix<T>(nbv, (int)qn * 6);
 					cp_async_6<T, P, 32>(d, g);
 				} else {
 					const T *g = p.btrace + ((long long)(-nbv - 1) * 6 + warp) * 6;
@@ -409,7 +380,7 @@ __device__ __forceinline__ void rk3_tile(const Rk3Params<T> &p, long long tile, 
 	if (live) {
 #pragma unroll
 		for (int j = 0; j < 10; j++)
-			w[j] = Wt[(j * 6 + c) * 32];
+			w[j] = Wt[rk3_off<T>(j, c)];
 	}
 	if (!FACT && live) {
 		const int d1 = (a + 1) % 3, d2 = (a + 2) % 3;
@@ -439,7 +410,7 @@ __device__ __forceinline__ void rk3_tile(const Rk3Params<T> &p, long long tile, 
 			T wL[6], vn[3], F[6];
 #pragma unroll
 			for (int cc = 0; cc < 6; cc++)
-				wL[cc] = Wt[(qo * 6 + cc) * 32];
+				wL[cc] = Wt[rk3_off<T>(qo, cc)];
 			// own scaled outward normal codtau . n_ref(f): the reference
 			// normals are -e_0, -e_1, -e_2 and (1,1,1)/sqrt(3), face 3 scaled by
 			// sqrt(3) (simulation.c:377-395; checked at attach)
@@ -470,11 +441,11 @@ __device__ __forceinline__ void rk3_tile(const Rk3Params<T> &p, long long tile, 
 		}
 	}
 	T k2o[10];
-	T *Kt = p.k2 + tile * 60 * 32 + lane;
+	T *Kt = p.k2 + tile * 60 * 32 + rk3_lane<T>(lane);
 	if (live && !p.stage0) {
 #pragma unroll
 		for (int i = 0; i < 10; i++)
-			k2o[i] = Kin[(i * 6 + c) * 32];
+			k2o[i] = Kin[rk3_off<T>(i, c)];
 	}
 
 	__syncthreads();
@@ -498,7 +469,7 @@ __device__ __forceinline__ void rk3_tile(const Rk3Params<T> &p, long long tile, 
 			T wf[10], v[4], t[4], cd[3];
 #pragma unroll
 			for (int j = 0; j < 10; j++)
-				wf[j] = Wt[(j * 6 + fld) * 32];
+				wf[j] = Wt[rk3_off<T>(j, fld)];
 			q4_apply_sym<T>(tb, wf, v, t);
 #pragma unroll
 			for (int k = 0; k < 3; k++)
@@ -550,13 +521,13 @@ __device__ __forceinline__ void rk3_tile(const Rk3Params<T> &p, long long tile, 
 		lift_minv_sym<T>(tb, R, dwv);
 	else
 		lift_minv<T>(tb, R, dwv);
-	T *Wo = p.w_out + tile * 60 * 32 + lane;
+	T *Wo = p.w_out + tile * 60 * 32 + rk3_lane<T>(lane);
 #pragma unroll
 	for (int i = 0; i < 10; i++) {
 		const T k2 = p.stage0 ? -(scale * dwv[i]) : A * k2o[i] - scale * dwv[i];
-		Wo[(i * 6 + c) * 32] = w[i] + B * k2;
+		Wo[rk3_off<T>(i, c)] = w[i] + B * k2;
 		if (p.write_k2)
-			Kt[(i * 6 + c) * 32] = k2;
+			Kt[rk3_off<T>(i, c)] = k2;
 	}
 }
 
@@ -591,10 +562,263 @@ __global__ void __launch_bounds__(kRk3Threads, MINB) rk3_stage_kernel(Rk3Params<
 			prefetch_l2(p.perm + tn * 32 * 4, nbb);
 		}
 	}
-	const T *Wt = p.w_in + tile * 60 * 32 + lane;
-	rk3_tile<T, SPARSE, FACT, PF, METAL>(p, tile, Wt, p.geom + tile * 10 * 32 + lane, p.k2 + tile * 60 * 32 + lane,
+	const T *Wt = p.w_in + tile * 60 * 32 + rk3_lane<T>(lane);
+	rk3_tile<T, SPARSE, FACT, PF, METAL>(p, tile, Wt, p.geom + tile * 10 * 32 + lane, p.k2 + tile * 60 * 32 + rk3_lane<T>(lane),
 										 reinterpret_cast<const int4 *>(p.nb) + ec,
 										 reinterpret_cast<const int4 *>(p.perm) + ec, sX, sF);
+}
+
+// FP32 stage kernel: a thread per element, a warp per tile, everything in
+// registers, no shared memory and no barrier.
+// The stage kernel above is bound by L1 wavefronts and instruction issue: its
+// six warps per tile exchange the fluxes through shared memory (432 rows) and
+// read the geometry six and the own state three times.  One thread that holds
+// all six fields of its element reads every value once, and the (E_c, H_c) pairs
+// of the layout make every step of the residual, which treats E and H alike,
+// packed FP32x2 arithmetic (the flux, the face mass, the derivatives, the lift
+// and the update): 64-bit rows instead of 32-bit ones, 2,250 instead of 6,670
+// warp instructions and 900 instead of 1,784 L1 wavefronts per tile and stage.
+// It is bound by the latency of its loads, so registers for loads in flight
+// count more than warps: 8 warps per SM at 222 registers beat 12 at 168.
+// ms per step, before / now: 48^3 0.556 / 0.354, 96^3 4.27 / 3.01 (4.6 TB/s of the
+// bytes that DRAM moves).
+constexpr int kElemThreads = 128;
+struct Rk3Elem {
+	static constexpr int lo = 2, hi = 3; // CTAs per SM: 255 / 168 registers
+};
+
+__device__ __forceinline__ float2 dup2(float a)
+{
+	return make_float2(a, a);
+}
+
+template <bool METAL, int MINB>
+__global__ void __launch_bounds__(kElemThreads, MINB) rk3_elem_kernel(Rk3Params<float> p)
+{
+	const Tables<float> &tb = tab<float>();
+	const int lane = threadIdx.x & 31;
+	const long long tile = blockIdx.x * (long long)(kElemThreads / 32) + (threadIdx.x >> 5);
+	const long long e = tile * 32 + lane;
+	if (e >= p.ne)
+		return;
+	if (lane == 0 && p.l2_ahead > 0) {
+		const long long tn = tile + p.l2_ahead;
+		if (tn * 32 < p.ne) {
+			prefetch_l2(p.w_in + tn * 1920, 7680);
+			if (!p.stage0)
+				prefetch_l2(p.k2 + tn * 1920, 7680);
+			prefetch_l2(p.geom + tn * 320, 1280);
+			const unsigned nbb = (unsigned)((p.ne - tn * 32 < 32 ? p.ne - tn * 32 : 32) * 16);
+			prefetch_l2(p.nb + tn * 128, nbb);
+			prefetch_l2(p.perm + tn * 128, nbb);
+		}
+	}
+	const float2 *W = reinterpret_cast<const float2 *>(p.w_in) + tile * 960 + lane;
+	const int4 nb4 = reinterpret_cast<const int4 *>(p.nb)[e];
+	const int4 pm4 = reinterpret_cast<const int4 *>(p.perm)[e];
+	float2 w[10][3], R[10][3];
+#pragma unroll
+	for (int i = 0; i < 10; i++)
+#pragma unroll
+		for (int a = 0; a < 3; a++)
+			w[i][a] = W[(i * 3 + a) * 32];
+	float cod[3][3];
+	const float *Gt = p.geom + tile * 320 + lane;
+#pragma unroll
+	for (int r = 0; r < 3; r++)
+#pragma unroll
+		for (int q = 0; q < 3; q++)
+			cod[r][q] = Gt[(3 * r + q) * 32];
+
+	// Neighbour traces, half a face (three vertices, then three edge nodes) at a
+	// time and half a face ahead of their use: component c of the face's node at
+	// g[off + c * st], with st and off those of a tile or of the boundary traces.
+	const int nbk[4] = {nb4.x, nb4.y, nb4.z, nb4.w}, pmk[4] = {pm4.x, pm4.y, pm4.z, pm4.w};
+	auto gather = [&](int fh, float2 r[3][3]) {
+		const int f = fh >> 1;
+		const int nbv = nbk[f];
+		const bool inner = nbv >= 0;
+		const float2 *g = inner ? reinterpret_cast<const float2 *>(p.w_in) + (long long)(nbv >> 5) * 960 + (nbv & 31)
+								: reinterpret_cast<const float2 *>(p.btrace) + (long long)(-nbv - 1) * 18;
+		const int st = inner ? 32 : 1;
+#pragma unroll
+		for (int j = 0; j < 3; j++) {
+			const int jj = 3 * (fh & 1) + j;
+			const float2 *gj = g + (inner ? ((pmk[f] >> (4 * jj)) & 15) * 96 : 3 * jj);
+#pragma unroll
+			for (int c = 0; c < 3; c++)
+				r[j][c] = __ldg(gj + c * st);
+		}
+	};
+	float2 wR[2][3][3];
+	gather(0, wR[0]);
+
+	// ---- curl: R_E += curl H, R_H -= curl E.  Component a of (H, -E) goes along
+	// direction a + 2 to component a + 1 and along a + 1, negated, to a + 2 ----
+#pragma unroll
+	for (int a = 0; a < 3; a++) {
+		// v = Q4 x, t = v - sum(v) / 4 (q4_apply_sym) of the pairs (E_a, H_a)
+		const float2 sv = __fadd2_rn(__fadd2_rn(w[0][a], w[1][a]), __fadd2_rn(w[2][a], w[3][a]));
+		const float2 se = __fadd2_rn(__fadd2_rn(__fadd2_rn(w[4][a], w[5][a]), __fadd2_rn(w[6][a], w[7][a])),
+									 __fadd2_rn(w[8][a], w[9][a]));
+		const float2 base = __ffma2_rn(dup2(tb.q4_sym[0]), sv, __fmul2_rn(dup2(tb.q4_sym[1]), se));
+		const float2 s = __ffma2_rn(dup2(tb.q4_sym[4]), sv, __fmul2_rn(dup2(tb.q4_sym[5]), se));
+		float2 v[4], t[4];
+#pragma unroll
+		for (int l = 0; l < 4; l++) {
+			float2 ev = make_float2(0.f, 0.f);
+			bool first = true;
+#pragma unroll
+			for (int ed = 0; ed < 6; ed++)
+				if (edge_end(ed, 0) == l || edge_end(ed, 1) == l) {
+					ev = first ? w[4 + ed][a] : __fadd2_rn(ev, w[4 + ed][a]);
+					first = false;
+				}
+			const float2 x =
+				__ffma2_rn(dup2(tb.q4_sym[3]), ev, __ffma2_rn(dup2(tb.q4_sym[2]), w[l][a], base));
+			v[l] = make_float2(x.y, -x.x); // (H, -E)
+			t[l] = make_float2(x.y - s.y, s.x - x.x);
+		}
+#pragma unroll
+		for (int h = 0; h < 2; h++) {
+			const int d = (a + 2 - h) % 3, to = (a + 1 + h) % 3; // direction, component of R
+			const float sg = h ? -1.f : 1.f;
+			const float g1 = sg * cod[d][0], g2 = sg * cod[d][1], g3 = sg * cod[d][2];
+			const float2 g[4] = {dup2(-(g1 + g2 + g3)), dup2(g1), dup2(g2), dup2(g3)};
+			// the first contribution to a component of R sets it: component 1 from
+			// a = 0 (h = 0), 2 from a = 0 (h = 1), 0 from a = 1 (h = 1)
+			const bool set = a == 0 || (a == 1 && h == 1);
+#pragma unroll
+			for (int i = 0; i < 4; i++)
+				R[i][to] = set ? __fmul2_rn(g[i], t[i]) : __ffma2_rn(g[i], t[i], R[i][to]);
+#pragma unroll
+			for (int ed = 0; ed < 6; ed++) {
+				const int i = edge_end(ed, 0), j = edge_end(ed, 1);
+				R[4 + ed][to] =
+					__ffma2_rn(g[i], v[j], set ? __fmul2_rn(g[j], v[i]) : __ffma2_rn(g[j], v[i], R[4 + ed][to]));
+			}
+		}
+	}
+
+	// ---- faces: R += S F, vertices then edges of the face ----
+	const float2 m1 = dup2(-1.f);
+#pragma unroll
+	for (int f = 0; f < 4; f++) {
+		const bool inner = nbk[f] >= 0;
+		float n[3];
+#pragma unroll
+		for (int a = 0; a < 3; a++)
+			n[a] = f < 3 ? -cod[a][f] : (cod[a][0] + cod[a][1] + cod[a][2]) * tb.n3scale;
+		const float rn = inv_norm_eps(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+		// F = h x u, u = m x d + (-s_H, s_E) with h = n / 2, m = n / |n|, d = wR - wL,
+		// s = wR + wL: upwind_flux_h with the double cross product factored
+#pragma unroll
+		for (int half = 0; half < 2; half++) {
+			float2 F[3][3];
+			if (2 * f + half < 7)
+				gather(2 * f + half + 1, wR[1 - half]);
+#pragma unroll
+			for (int j = 0; j < 3; j++) {
+				const int qo = f2n(f, 3 * half + j);
+				float2 d[3], q[3];
+#pragma unroll
+				for (int a = 0; a < 3; a++) {
+					float2 r = wR[half][j][a];
+					if (METAL && !inner)
+						r = w[qo][a]; // no jump: F_E = -n x H_L, F_H set to zero below
+					d[a] = __ffma2_rn(w[qo][a], m1, r);
+					q[a] = make_float2(-(r.y + w[qo][a].y), r.x + w[qo][a].x);
+				}
+				float2 u[3];
+#pragma unroll
+				for (int a = 0; a < 3; a++) {
+					const int b = (a + 1) % 3, c = (a + 2) % 3;
+					u[a] = __ffma2_rn(dup2(n[b] * rn), d[c], __ffma2_rn(dup2(-n[c] * rn), d[b], q[a]));
+				}
+#pragma unroll
+				for (int a = 0; a < 3; a++) {
+					const int b = (a + 1) % 3, c = (a + 2) % 3;
+					F[j][a] = __ffma2_rn(dup2(0.5f * n[b]), u[c], __fmul2_rn(dup2(-0.5f * n[c]), u[b]));
+					if (METAL && !inner)
+						F[j][a].y = 0.f;
+				}
+			}
+			const float2 s_own = dup2(tb.s_sym[half ? 3 : 0]), s_all = dup2(tb.s_sym[half ? 4 : 1]),
+						 s_opp = dup2(tb.s_sym[2]);
+#pragma unroll
+			for (int a = 0; a < 3; a++) {
+				const float2 sum = __fmul2_rn(s_all, __fadd2_rn(__fadd2_rn(F[0][a], F[1][a]), F[2][a]));
+#pragma unroll
+				for (int j = 0; j < 3; j++) {
+					// face-local vertex j is opposite the edge 3 + (j + 1) % 3
+					const int own = f2n(f, 3 * half + j), opp = f2n(f, half ? (j + 2) % 3 : 3 + (j + 1) % 3);
+					R[own][a] = __fadd2_rn(R[own][a], __ffma2_rn(s_own, F[j][a], sum));
+					R[opp][a] = __ffma2_rn(s_opp, F[j][a], R[opp][a]);
+				}
+			}
+		}
+	}
+
+	// ---- lift (lift_minv_sym) and RK update ----
+	const float dt = p.einst ? (float)p.dt_tab[p.einst[e]] : (float)p.dt;
+	const float2 A = dup2((float)p.A), B = dup2((float)p.B), scale = dup2(-(dt / Gt[9 * 32]));
+	float2 *K = reinterpret_cast<float2 *>(p.k2) + tile * 960 + lane;
+	float2 *Wo = reinterpret_cast<float2 *>(p.w_out) + tile * 960 + lane;
+	// k2 of a component is read before the stores of the one before it: the
+	// compiler moves no load over a store, and 30 loads behind one another cost
+	// as much as the rest of the stage
+	float2 ko[10];
+	if (!p.stage0) {
+#pragma unroll
+		for (int i = 0; i < 10; i++)
+			ko[i] = K[i * 96];
+	}
+#pragma unroll
+	for (int a = 0; a < 3; a++) {
+		const float2 sv = __fadd2_rn(__fadd2_rn(R[0][a], R[1][a]), __fadd2_rn(R[2][a], R[3][a]));
+		const float2 se = __fadd2_rn(__fadd2_rn(__fadd2_rn(R[4][a], R[5][a]), __fadd2_rn(R[6][a], R[7][a])),
+									 __fadd2_rn(R[8][a], R[9][a]));
+		const float2 bv = __ffma2_rn(dup2(tb.minv_sym[0]), sv, __fmul2_rn(dup2(tb.minv_sym[1]), se));
+		const float2 be = __ffma2_rn(dup2(tb.minv_sym[1]), sv, __fmul2_rn(dup2(tb.minv_sym[2]), se));
+		float2 ev[4];
+#pragma unroll
+		for (int l = 0; l < 4; l++) {
+			bool first = true;
+#pragma unroll
+			for (int ed = 0; ed < 6; ed++)
+				if (edge_end(ed, 0) == l || edge_end(ed, 1) == l) {
+					ev[l] = first ? R[4 + ed][a] : __fadd2_rn(ev[l], R[4 + ed][a]);
+					first = false;
+				}
+		}
+		float2 kn[10];
+#pragma unroll
+		for (int i = 0; i < 10; i++) {
+			float2 dw;
+			if (i < 4) {
+				dw = __ffma2_rn(dup2(tb.minv_sym[4]), ev[i], __ffma2_rn(dup2(tb.minv_sym[3]), R[i][a], bv));
+			} else {
+				const int l = edge_end(i - 4, 0), m = edge_end(i - 4, 1);
+				dw = __ffma2_rn(dup2(tb.minv_sym[4]), __fadd2_rn(R[l][a], R[m][a]), be);
+				dw = __ffma2_rn(dup2(tb.minv_sym[5]), R[i][a], dw);
+				dw = __ffma2_rn(dup2(tb.minv_sym[6]), __fadd2_rn(ev[l], ev[m]), dw);
+			}
+			kn[i] = __fmul2_rn(scale, dw);
+			if (!p.stage0)
+				kn[i] = __ffma2_rn(A, ko[i], kn[i]);
+		}
+		if (!p.stage0 && a < 2) {
+#pragma unroll
+			for (int i = 0; i < 10; i++)
+				ko[i] = K[(i * 3 + a + 1) * 32];
+		}
+#pragma unroll
+		for (int i = 0; i < 10; i++) {
+			Wo[(i * 3 + a) * 32] = __ffma2_rn(B, kn[i], w[i][a]);
+			if (p.write_k2)
+				K[(i * 3 + a) * 32] = kn[i];
+		}
+	}
 }
 
 // P2 structural-zero pattern check for the tables handed to attach.
@@ -801,10 +1025,12 @@ static int prepare_rk3_one()
 template <typename T>
 int prepare_rk3()
 {
-	GDN_RK3_TRY((prepare_rk3_one<T, true, true, false>()));
+	if constexpr (sizeof(T) == 8) {
+		GDN_RK3_TRY((prepare_rk3_one<T, true, true, false>()));
+		GDN_RK3_TRY((prepare_rk3_one<T, true, true, true>()));
+	}
 	GDN_RK3_TRY((prepare_rk3_one<T, true, false, false>()));
 	GDN_RK3_TRY((prepare_rk3_one<T, false, false, false>()));
-	GDN_RK3_TRY((prepare_rk3_one<T, true, true, true>()));
 	GDN_RK3_TRY((prepare_rk3_one<T, true, false, true>()));
 	GDN_RK3_TRY((prepare_rk3_one<T, false, false, true>()));
 	return GDN_CUDA_OK;
@@ -829,12 +1055,30 @@ static void launch_rk3_one(const Rk3Params<T> &pin, int variant, cudaStream_t s)
 		rk3_stage_kernel<T, SP, FA, V::hi, V::pf_hi, METAL><<<nblk, kRk3Threads, sm, s>>>(p);
 }
 
+template <bool METAL>
+static void launch_rk3_elem(const Rk3Params<float> &pin, int variant, cudaStream_t s)
+{
+	Rk3Params<float> p = pin;
+	constexpr int tiles = kElemThreads / 32;
+	// a quarter of the resident tiles ahead (ms per step for none, 1/4, 1/2, 1 and
+	// 1.5 times: 48^3 0.405, 0.354, 0.368, 0.382, 0.428; 96^3 3.06, 3.01, 3.02, 3.00, 3.45)
+	p.l2_ahead = p.l2_ahead ? p.num_sms * (variant == 0 ? Rk3Elem::lo : Rk3Elem::hi) : 0;
+	const unsigned nblk = (unsigned)(((p.ne + 31) / 32 + tiles - 1) / tiles);
+	if (variant == 0)
+		rk3_elem_kernel<METAL, Rk3Elem::lo><<<nblk, kElemThreads, 0, s>>>(p);
+	else
+		rk3_elem_kernel<METAL, Rk3Elem::hi><<<nblk, kElemThreads, 0, s>>>(p);
+}
+
 template <typename T, bool METAL>
 static void launch_rk3_tables(const Rk3Params<T> &p, int variant, cudaStream_t s)
 {
-	if (p.sparse && p.fact)
-		launch_rk3_one<T, true, true, METAL>(p, variant, s);
-	else if (p.sparse)
+	if (p.sparse && p.fact) {
+		if constexpr (sizeof(T) == 4)
+			launch_rk3_elem<METAL>(p, variant, s);
+		else
+			launch_rk3_one<T, true, true, METAL>(p, variant, s);
+	} else if (p.sparse)
 		launch_rk3_one<T, true, false, METAL>(p, variant, s);
 	else
 		launch_rk3_one<T, false, false, METAL>(p, variant, s);
@@ -852,10 +1096,12 @@ int launch_rk3_stage(const Rk3Params<T> &p, int variant, cudaStream_t s)
 	return GDN_CUDA_OK;
 }
 
-int rk3_min_blocks(int precision_fp64, int variant)
+int rk3_min_blocks(int precision_fp64, int fact, int variant)
 {
 	if (precision_fp64)
 		return variant == 0 ? Rk3Variants<double>::lo : Rk3Variants<double>::hi;
+	if (fact)
+		return variant == 0 ? Rk3Elem::lo : Rk3Elem::hi;
 	return variant == 0 ? Rk3Variants<float>::lo : Rk3Variants<float>::hi;
 }
 
@@ -869,7 +1115,7 @@ __global__ void rk3_to_tiles_kernel(const double *__restrict__ src, T *__restric
 		return;
 	const long long e = u / 60;
 	const int k = (int)(u % 60);
-	dst[rk3_tix(e0 + e, k)] = (T)src[u];
+	dst[rk3_tix<T>(e0 + e, k)] = (T)src[u];
 }
 template <typename T>
 __global__ void rk3_from_tiles_kernel(const T *__restrict__ src, double *__restrict__ dst, long long e0, long long ne)
@@ -879,7 +1125,7 @@ __global__ void rk3_from_tiles_kernel(const T *__restrict__ src, double *__restr
 		return;
 	const long long e = u / 60;
 	const int k = (int)(u % 60);
-	dst[u] = (double)src[rk3_tix(e0 + e, k)];
+	dst[u] = (double)src[rk3_tix<T>(e0 + e, k)];
 }
 // geometry [e][10] FP64 -> tiles of T
 template <typename T>
