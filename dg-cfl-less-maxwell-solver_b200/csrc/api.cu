@@ -97,7 +97,7 @@ struct gdn_cuda_handle {
 	// RK3
 	void *w[2] = {nullptr, nullptr};
 	void *k2 = nullptr;
-	void *btrace = nullptr; // [nbf][6][6] boundary traces at the stage time
+	void *btrace = nullptr; // [2][3][nbf][6][6] boundary traces of the three stages, by step parity (cur)
 	int cur = 0;
 	int rk3_variant = 0; // stage kernel for fewer (0) / more (1) resident CTAs per SM
 	bool rk3_autotune = true; // pick the variant at attach by timing both
@@ -130,11 +130,11 @@ struct gdn_cuda_handle {
 	int *level_off_dev = nullptr;
 	unsigned *bar = nullptr; // [2] grid barrier of the cooperative sweep
 	int *err = nullptr; // set on the device when a barrier wait gave up
-	int *items = nullptr; // [k] e * nv + v
-	int *pos = nullptr; // [e * nv + v] k
+	int *items = nullptr; // kinetic: [k] e * nv + v; RK3: [k] element at position k
+	int *pos = nullptr; // kinetic: [e * nv + v] k; RK3: [e] position in the device order
 	std::vector<int> level_off;
 	// device time and captured step loops
-	double *t_dev = nullptr; // [ninst]
+	double *t_dev = nullptr; // [ninst]; RK3 [2][ninst], by step parity (cur)
 	cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};
 	long long graph_nodes[2] = {0, 0};
 	// batch of instances: concatenated meshes, per-instance dt / data / time.
@@ -435,6 +435,7 @@ static int autotune_rk3(gdn_cuda_handle *h)
 	p.idx32 = (h->ne + 31) / 32 * 1920 <= 0xffffffffLL;
 	p.l2_ahead = 1;
 	p.bc_metal = h->bc_metal;
+	p.traces = 0;
 	cudaEvent_t ev[2];
 	GDN_CUDA_TRY(cudaEventCreate(&ev[0]));
 	GDN_CUDA_TRY(cudaEventCreate(&ev[1]));
@@ -510,7 +511,7 @@ static int attach_impl(gdn_cuda_handle *h, const gdn_cuda_mesh *m, const gdn_cud
 	h->nblk_err = 1184; // 8 x 148 SMs
 	GDN_TRY(dalloc(h, &h->partial, 6 * h->nblk_err));
 	GDN_TRY(dalloc(h, &h->result, 8));
-	GDN_TRY(dalloc(h, &h->t_dev, h->ninst));
+	GDN_TRY(dalloc(h, &h->t_dev, 2 * h->ninst));
 	GDN_TRY(dalloc(h, &h->dt_dev, h->ninst));
 	GDN_TRY(dalloc(h, &h->data_dev, h->ninst));
 	GDN_CUDA_TRY(cudaMallocHost(&h->host_result, 8 * sizeof(double)));
@@ -553,24 +554,34 @@ static int attach_impl(gdn_cuda_handle *h, const gdn_cuda_mesh *m, const gdn_cud
 		// state, k2 and geometry in tiles of 32 elements (the last one padded)
 		const long long nt = 32 * ((ne + 31) / 32);
 		h->neq = 10 * ne + 6 * nbf;
+		// the device order, and the neighbour rows in it (the staging buffer holds
+		// the rows in the mesh's order meanwhile)
+		GDN_TRY(dalloc(h, &h->staging, 6 * h->neq));
+		GDN_TRY(dalloc(h, &h->pos, ne));
+		GDN_TRY(dalloc(h, &h->items, ne));
+		int *raw = reinterpret_cast<int *>(h->staging);
+		GDN_CUDA_TRY(cudaMemcpyAsync(raw, h->nb, 4 * ne * sizeof(int), cudaMemcpyDeviceToDevice, s));
+		GDN_CUDA_TRY(cudaMemcpyAsync(raw + 4 * ne, h->perm, 4 * ne * sizeof(int), cudaMemcpyDeviceToDevice, s));
+		GDN_TRY(launch_rk3_order(h->e2q, h->einst, raw, raw + 4 * ne, ne, h->pos, h->items, h->nb, h->perm, s));
+		h->launches += 2;
 		if (fp64) {
 			double *gt;
 			GDN_TRY(dalloc(h, &gt, 10 * nt));
-			GDN_TRY(launch_geom_to_tiles<double>(h->geom64, gt, ne, s));
+			GDN_TRY(launch_geom_to_tiles<double>(h->geom64, gt, h->pos, ne, s));
 			h->geomT = gt;
 		} else {
 			float *gt;
 			GDN_TRY(dalloc(h, &gt, 10 * nt));
-			GDN_TRY(launch_geom_to_tiles<float>(h->geom64, gt, ne, s));
+			GDN_TRY(launch_geom_to_tiles<float>(h->geom64, gt, h->pos, ne, s));
 			h->geomT = gt;
 		}
 		h->launches++;
 		GDN_TRY(prepare_rk3<double>());
 		GDN_TRY(prepare_rk3<float>());
 		if (fp64)
-			GDN_TRY(dalloc(h, reinterpret_cast<double **>(&h->btrace), 36 * (nbf > 0 ? nbf : 1)));
+			GDN_TRY(dalloc(h, reinterpret_cast<double **>(&h->btrace), 216 * (nbf > 0 ? nbf : 1)));
 		else
-			GDN_TRY(dalloc(h, reinterpret_cast<float **>(&h->btrace), 36 * (nbf > 0 ? nbf : 1)));
+			GDN_TRY(dalloc(h, reinterpret_cast<float **>(&h->btrace), 216 * (nbf > 0 ? nbf : 1)));
 		for (int b = 0; b < 2; b++) {
 			if (fp64)
 				GDN_TRY(dalloc(h, reinterpret_cast<double **>(&h->w[b]), 60 * nt));
@@ -582,10 +593,9 @@ static int attach_impl(gdn_cuda_handle *h, const gdn_cuda_mesh *m, const gdn_cud
 		else
 			GDN_TRY(dalloc(h, reinterpret_cast<float **>(&h->k2), 60 * nt));
 		GDN_CUDA_TRY(cudaMemsetAsync(h->k2, 0, 60 * nt * h->ssize, s));
-		GDN_TRY(dalloc(h, &h->staging, 6 * h->neq));
 		if (h->rk3_autotune) {
 			GDN_CUDA_TRY(cudaMemsetAsync(h->w[0], 0, 60 * nt * h->ssize, s));
-			GDN_CUDA_TRY(cudaMemsetAsync(h->btrace, 0, 36 * (nbf > 0 ? nbf : 1) * h->ssize, s));
+			GDN_CUDA_TRY(cudaMemsetAsync(h->btrace, 0, 216 * (nbf > 0 ? nbf : 1) * h->ssize, s));
 			if (fp64)
 				GDN_TRY(autotune_rk3<double>(h));
 			else
@@ -932,10 +942,26 @@ extern "C" int gdn_cuda_detach(gdn_cuda_handle *h)
 // ------------------------------------------------------------ stepping --
 
 // ---- enqueue one time step (no host bookkeeping; capturable) ----
+// the boundary traces of the step of parity `par`; advance: of the step after
+// the one whose time is in slot 1 - par
+template <typename T>
+static Rk3Trace<T> rk3_traces(gdn_cuda_handle *h, int par, int advance)
+{
+	Rk3Trace<T> tr;
+	tr.bxyz = h->bxyz;
+	tr.nbf = h->nbf;
+	tr.b = h->batch();
+	tr.t_in = h->t_dev + (advance ? 1 - par : par) * h->ninst;
+	tr.t_out = h->t_dev + par * h->ninst;
+	tr.out = as<T>(h->btrace) + (long long)par * 108 * h->nbf;
+	tr.advance = advance;
+	return tr;
+}
+
 template <typename T>
 static int rk3_enqueue(gdn_cuda_handle *h, int &cur, long long &nlaunch)
 {
-	const Batch bt = h->batch();
+	const int par = cur; // a step flips cur three times
 	for (int i = 0; i < 3; i++) {
 		Rk3Params<T> p;
 		p.w_in = as<T>(h->w[cur]);
@@ -944,7 +970,7 @@ static int rk3_enqueue(gdn_cuda_handle *h, int &cur, long long &nlaunch)
 		p.geom = reinterpret_cast<const T *>(h->geomT);
 		p.nb = h->nb;
 		p.perm = h->perm;
-		p.btrace = as<T>(h->btrace);
+		p.btrace = as<T>(h->btrace) + (par * 3LL + i) * 36 * h->nbf;
 		p.einst = h->einst;
 		p.dt_tab = h->dt_dev;
 		p.ne = h->ne;
@@ -959,16 +985,12 @@ static int rk3_enqueue(gdn_cuda_handle *h, int &cur, long long &nlaunch)
 		p.idx32 = (h->ne + 31) / 32 * 1920 <= 0xffffffffLL;
 		p.l2_ahead = 1;
 		p.bc_metal = h->bc_metal;
-		if (h->nbf > 0) {
-			GDN_TRY(launch_boundary_trace<T>(h->bxyz, h->nbf, bt, RK_C[i], as<T>(h->btrace), h->stream));
-			nlaunch++;
-		}
+		p.traces = i == 2;
+		p.tr = rk3_traces<T>(h, 1 - par, 1);
 		GDN_TRY(launch_rk3_stage<T>(p, h->rk3_variant, h->stream));
 		nlaunch++;
 		cur = 1 - cur;
 	}
-	GDN_TRY(launch_advance_time(bt, h->stream));
-	nlaunch++;
 	return GDN_CUDA_OK;
 }
 
@@ -1398,6 +1420,22 @@ static int kin_pack(gdn_cuda_handle *h, int i, int to_ref)
 	return launch_kin_pack<__nv_bfloat16>(as<__nv_bfloat16>(h->f), pos, ne, h->nv, neq, st, to_ref, h->stream);
 }
 
+// the device time of every instance and, for RK3 (cur = 0), the boundary traces
+// of the step that starts there
+static int set_device_time(gdn_cuda_handle *h, double t)
+{
+	GDN_TRY(launch_set_time(h->batch(), t, h->stream));
+	h->launches++;
+	if (h->scheme == GDN_CUDA_SCHEME_RK3) {
+		if (h->precision == GDN_CUDA_FP64)
+			GDN_TRY(launch_rk3_traces<double>(rk3_traces<double>(h, 0, 0), h->stream));
+		else
+			GDN_TRY(launch_rk3_traces<float>(rk3_traces<float>(h, 0, 0), h->stream));
+		h->launches++;
+	}
+	return GDN_CUDA_OK;
+}
+
 // dg_init_sol_macro (dg.c:32-59) of every instance with its own data
 extern "C" int gdn_cuda_init(gdn_cuda_handle *h)
 {
@@ -1412,9 +1450,9 @@ extern "C" int gdn_cuda_init(gdn_cuda_handle *h)
 		const Data &d = h->hdata[i];
 		if (h->scheme == GDN_CUDA_SCHEME_RK3) {
 			if (h->precision == GDN_CUDA_FP64)
-				GDN_TRY(launch_init_rk3<double>(e2q, h->node, ne, e0, d, as<double>(h->w[0]), s));
+				GDN_TRY(launch_init_rk3<double>(h->e2q, h->node, e0, ne, h->items, d, as<double>(h->w[0]), s));
 			else
-				GDN_TRY(launch_init_rk3<float>(e2q, h->node, ne, e0, d, as<float>(h->w[0]), s));
+				GDN_TRY(launch_init_rk3<float>(h->e2q, h->node, e0, ne, h->items, d, as<float>(h->w[0]), s));
 		} else {
 			const int *pos = h->pos + e0 * h->nv;
 			if (sk == 0)
@@ -1430,8 +1468,7 @@ extern "C" int gdn_cuda_init(gdn_cuda_handle *h)
 		h->cur = 0;
 		GDN_CUDA_TRY(cudaMemsetAsync(h->k2, 0, 60 * 32 * ((h->ne + 31) / 32) * h->ssize, s));
 	}
-	GDN_TRY(launch_set_time(h->batch(), 0.0, s));
-	h->launches++;
+	GDN_TRY(set_device_time(h, 0.0));
 	h->ht.assign(h->ninst, 0.0);
 	h->ht_bdof.assign(h->ninst, 0.0);
 	h->steps = 0;
@@ -1455,9 +1492,9 @@ extern "C" int gdn_cuda_set_state(gdn_cuda_handle *h, const double *wn, double t
 			double *st = h->staging + h->w_off[i];
 			GDN_CUDA_TRY(cudaMemcpyAsync(st, src, 60 * ne * sizeof(double), cudaMemcpyHostToDevice, s));
 			if (h->precision == GDN_CUDA_FP64)
-				GDN_TRY(launch_rk3_to_tiles<double>(st, as<double>(h->w[0]), e0, ne, s));
+				GDN_TRY(launch_rk3_to_tiles<double>(st, as<double>(h->w[0]), h->pos + e0, ne, s));
 			else
-				GDN_TRY(launch_rk3_to_tiles<float>(st, as<float>(h->w[0]), e0, ne, s));
+				GDN_TRY(launch_rk3_to_tiles<float>(st, as<float>(h->w[0]), h->pos + e0, ne, s));
 			h->launches++;
 		}
 		GDN_CUDA_TRY(cudaMemsetAsync(h->k2, 0, 60 * 32 * ((h->ne + 31) / 32) * h->ssize, s));
@@ -1468,8 +1505,7 @@ extern "C" int gdn_cuda_set_state(gdn_cuda_handle *h, const double *wn, double t
 			h->launches++;
 		}
 	}
-	GDN_TRY(launch_set_time(h->batch(), t, s));
-	h->launches++;
+	GDN_TRY(set_device_time(h, t));
 	h->ht.assign(h->ninst, t);
 	h->ht_bdof.assign(h->ninst, t);
 	return GDN_CUDA_OK;
@@ -1491,9 +1527,9 @@ static int get_state_impl(gdn_cuda_handle *h, double *wn)
 										 st + 60 * ne, s));
 			h->launches++;
 			if (h->precision == GDN_CUDA_FP64)
-				GDN_TRY(launch_rk3_from_tiles<double>(as<double>(h->w[h->cur]), st, e0, ne, s));
+				GDN_TRY(launch_rk3_from_tiles<double>(as<double>(h->w[h->cur]), st, h->pos + e0, ne, s));
 			else
-				GDN_TRY(launch_rk3_from_tiles<float>(as<float>(h->w[h->cur]), st, e0, ne, s));
+				GDN_TRY(launch_rk3_from_tiles<float>(as<float>(h->w[h->cur]), st, h->pos + e0, ne, s));
 			h->launches++;
 			GDN_CUDA_TRY(cudaMemcpyAsync(dst, st, 60 * ne * sizeof(double), cudaMemcpyDeviceToHost, s));
 			if (nbf > 0)
@@ -1558,21 +1594,20 @@ static int error_l2_impl(gdn_cuda_handle *h, int i, double *err)
 	const bool kin = h->scheme == GDN_CUDA_SCHEME_KINETIC;
 	const int sk = kin ? kin_state_kind(h) : (h->precision == GDN_CUDA_FP64 ? 0 : 1);
 	const long long e0 = h->e_off[i], ne = h->e_off[i + 1] - e0;
-	const long long te0 = kin ? 0 : e0; // RK3: tiled state indexed by global element; kinetic: through pos
-	const int *pos = kin ? h->pos + e0 * h->nv : nullptr;
+	const int *pos = h->pos + e0 * (kin ? h->nv : 1);
 	const int *e2q = h->e2q + 10 * e0;
 	const double *geom = h->geom64 + 10 * e0;
 	void *st = kin ? h->f : h->w[h->cur];
 	const double t = h->ht[i];
 	const Data &d = h->hdata[i];
 	if (sk == 0)
-		GDN_TRY(launch_error_l2<double>(as<double>(st), kin, te0, h->nv, pos, e2q, h->node, geom, ne, d, t,
+		GDN_TRY(launch_error_l2<double>(as<double>(st), kin, h->nv, pos, e2q, h->node, geom, ne, d, t,
 										h->partial, h->nblk_err, h->result, s));
 	else if (sk == 1)
-		GDN_TRY(launch_error_l2<float>(as<float>(st), kin, te0, h->nv, pos, e2q, h->node, geom, ne, d, t, h->partial,
+		GDN_TRY(launch_error_l2<float>(as<float>(st), kin, h->nv, pos, e2q, h->node, geom, ne, d, t, h->partial,
 									   h->nblk_err, h->result, s));
 	else
-		GDN_TRY(launch_error_l2<__nv_bfloat16>(as<__nv_bfloat16>(st), kin, te0, h->nv, pos, e2q, h->node, geom, ne, d,
+		GDN_TRY(launch_error_l2<__nv_bfloat16>(as<__nv_bfloat16>(st), kin, h->nv, pos, e2q, h->node, geom, ne, d,
 											   t, h->partial, h->nblk_err, h->result, s));
 	h->launches += 2;
 	GDN_CUDA_TRY(cudaMemcpyAsync(h->host_result, h->result, 7 * sizeof(double), cudaMemcpyDeviceToHost, s));

@@ -79,36 +79,38 @@ __device__ __forceinline__ void node_xyz(const int *e2q, const double *node, lon
 	x[2] = node[3 * q + 2];
 }
 
-// dg_init_sol_macro, RK3 branch (src/dg/dg.c:32-59): w = w_exact(x, 0) for
-// the elements e0 .. e0 + ne - 1 (e2q points at element e0), tiled layout
+// dg_init_sol_macro, RK3 branch (src/dg/dg.c:32-59): w = w_exact(x, 0) of the
+// elements at the positions k0 .. k0 + ne - 1 of the tiled layout (items[k]: the
+// element there), a lane per position so that the rows are written whole
 template <typename S>
-__global__ void init_rk3_kernel(const int *__restrict__ e2q, const double *__restrict__ node, long long ne,
-								long long e0, Data d, S *__restrict__ w)
+__global__ void init_rk3_kernel(const int *__restrict__ e2q, const double *__restrict__ node, long long k0,
+								long long ne, const int *__restrict__ items, Data d, S *__restrict__ w)
 {
 	const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-	if (t >= ne * 10)
+	const long long k = (k0 & ~31LL) + t / 320 * 32 + (t & 31);
+	if (k < k0 || k >= k0 + ne)
 		return;
-	const long long e = t / 10;
-	const int i = (int)(t % 10);
+	const int i = (int)(t / 32 % 10);
 	double x[3], we[6];
-	node_xyz(e2q, node, e, i, x);
+	node_xyz(e2q, node, items[k], i, x);
 	exact_w(d, x, 0.0, we);
 	for (int c = 0; c < 6; c++)
-		Store<S>::store(w + rk3_tix<S>(e0 + e, i * 6 + c), we[c]);
+		Store<S>::store(w + rk3_tix<S>(k, i * 6 + c), we[c]);
 }
 
 template <typename S>
-int launch_init_rk3(const int *e2q, const double *node, long long ne, long long e0, const Data &d, S *w,
-					cudaStream_t s)
+int launch_init_rk3(const int *e2q, const double *node, long long k0, long long ne, const int *items, const Data &d,
+					S *w, cudaStream_t s)
 {
-	init_rk3_kernel<S><<<(unsigned)((ne * 10 + 255) / 256), 256, 0, s>>>(e2q, node, ne, e0, d, w);
+	const long long n = ((k0 + ne - 1) / 32 - k0 / 32 + 1) * 320;
+	init_rk3_kernel<S><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(e2q, node, k0, ne, items, d, w);
 	GDN_CUDA_TRY(cudaGetLastError());
 	return GDN_CUDA_OK;
 }
-template int launch_init_rk3<double>(const int *, const double *, long long, long long, const Data &, double *,
-									 cudaStream_t);
-template int launch_init_rk3<float>(const int *, const double *, long long, long long, const Data &, float *,
-									cudaStream_t);
+template int launch_init_rk3<double>(const int *, const double *, long long, long long, const int *, const Data &,
+									 double *, cudaStream_t);
+template int launch_init_rk3<float>(const int *, const double *, long long, long long, const int *, const Data &,
+									float *, cudaStream_t);
 
 // f_eq of the kinetic model: f_v = w / nv + feq_c A(v) w
 __device__ __forceinline__ void feq_component(const double w[6], const double *v, int nv, double feq_c,
@@ -180,39 +182,6 @@ __global__ void boundary_dofs_kernel(const double *__restrict__ bxyz, long long 
 		}
 	}
 }
-
-// RK3 boundary traces at a stage time, in the stage kernels' precision:
-// out[(bf*6 + jj)*6 + rk3_btrace_off(c)] = w_exact(x_{bf,jj}, t)_c  (dg_update_boundary,
-// dg.c:101-104, evaluated once per stage instead of inside the flux loop),
-// with the data, time and time step of the face's instance.  The stage time
-// t + C_i dt is formed from the device copy of t with the host's rounding (no
-// fused multiply-add), so every stage sees the reference's time bits.
-template <typename T>
-__global__ void boundary_trace_kernel(const double *__restrict__ bxyz, long long nbf, Batch b, double c_stage,
-									  T *__restrict__ out)
-{
-	const long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-	if (u >= nbf * 6)
-		return;
-	const int inst = b.bfinst ? b.bfinst[u / 6] : 0;
-	const double t = __dadd_rn(b.t[inst], __dmul_rn(c_stage, b.dt[inst]));
-	double x[3] = {bxyz[3 * u], bxyz[3 * u + 1], bxyz[3 * u + 2]}, we[6];
-	exact_w(b.data[inst], x, t, we);
-	for (int c = 0; c < 6; c++)
-		out[u * 6 + rk3_btrace_off<T>(c)] = (T)we[c];
-}
-
-template <typename T>
-int launch_boundary_trace(const double *bxyz, long long nbf, const Batch &b, double c_stage, T *out, cudaStream_t s)
-{
-	if (nbf <= 0)
-		return GDN_CUDA_OK;
-	boundary_trace_kernel<T><<<(unsigned)((nbf * 6 + 255) / 256), 256, 0, s>>>(bxyz, nbf, b, c_stage, out);
-	GDN_CUDA_TRY(cudaGetLastError());
-	return GDN_CUDA_OK;
-}
-template int launch_boundary_trace<double>(const double *, long long, const Batch &, double, double *, cudaStream_t);
-template int launch_boundary_trace<float>(const double *, long long, const Batch &, double, float *, cudaStream_t);
 
 // device time of every instance: t = value, and t += dt (the reference's
 // accumulation, explicit.c:103 / relaxation.c:171)
@@ -317,7 +286,7 @@ template int launch_kin_pack<__nv_bfloat16>(const __nv_bfloat16 *, const int *, 
 // FP64 partial per block and field, in a fixed order; pass 2: one block sums
 // the partials in order.  Deterministic for a given launch shape.
 template <typename S>
-__global__ void error_partial_kernel(const S *__restrict__ state, int kinetic, long long e0, int nv,
+__global__ void error_partial_kernel(const S *__restrict__ state, int kinetic, int nv,
 									 const int *__restrict__ pos,
 									 const int *__restrict__ e2q, const double *__restrict__ node,
 									 const double *__restrict__ geom, long long ne, Data d, double t,
@@ -335,7 +304,7 @@ __global__ void error_partial_kernel(const S *__restrict__ state, int kinetic, l
 		exact_w(d, x, t, we);
 		if (!kinetic) {
 			for (int c = 0; c < 6; c++)
-				wl[c] = (double)Store<S>::load(state + rk3_tix<S>(e0 + e, i * 6 + c));
+				wl[c] = (double)Store<S>::load(state + rk3_tix<S>(pos[e], i * 6 + c));
 		} else {
 			for (int c = 0; c < 6; c++) {
 				double s = 0.0;
@@ -391,23 +360,23 @@ __global__ void error_final_kernel(const double *__restrict__ partial, int nblk,
 }
 
 template <typename S>
-int launch_error_l2(const S *state, int kinetic, long long e0, int nv, const int *pos, const int *e2q,
+int launch_error_l2(const S *state, int kinetic, int nv, const int *pos, const int *e2q,
 					const double *node, const double *geom, long long ne, const Data &d, double t, double *partial,
 					int nblk, double *out, cudaStream_t s)
 {
-	error_partial_kernel<S><<<nblk, 256, 0, s>>>(state, kinetic, e0, nv, pos, e2q, node, geom, ne, d, t, partial);
+	error_partial_kernel<S><<<nblk, 256, 0, s>>>(state, kinetic, nv, pos, e2q, node, geom, ne, d, t, partial);
 	GDN_CUDA_TRY(cudaGetLastError());
 	error_final_kernel<<<1, 256, 0, s>>>(partial, nblk, out);
 	GDN_CUDA_TRY(cudaGetLastError());
 	return GDN_CUDA_OK;
 }
-template int launch_error_l2<double>(const double *, int, long long, int, const int *, const int *, const double *,
+template int launch_error_l2<double>(const double *, int, int, const int *, const int *, const double *,
 									 const double *, long long, const Data &, double, double *, int, double *,
 									 cudaStream_t);
-template int launch_error_l2<float>(const float *, int, long long, int, const int *, const int *, const double *,
+template int launch_error_l2<float>(const float *, int, int, const int *, const int *, const double *,
 									const double *, long long, const Data &, double, double *, int, double *,
 									cudaStream_t);
-template int launch_error_l2<__nv_bfloat16>(const __nv_bfloat16 *, int, long long, int, const int *, const int *,
+template int launch_error_l2<__nv_bfloat16>(const __nv_bfloat16 *, int, int, const int *, const int *,
 											const double *, const double *, long long, const Data &, double, double *,
 											int, double *, cudaStream_t);
 
@@ -440,7 +409,7 @@ __global__ void io_values_kernel(const S *__restrict__ st, int kinetic, int nv, 
 	const int i = u % 10;
 	if (!kinetic) {
 		for (int c = 0; c < 6; c++)
-			out[c * nq + in] = (double)Store<S>::load(st + rk3_tix<S>(e, i * 6 + c));
+			out[c * nq + in] = (double)Store<S>::load(st + rk3_tix<S>(pos[e], i * 6 + c));
 	} else {
 		// component im = iw * nv + iv of the reference's kinetic wn
 		for (int v = 0; v < nv; v++) {

@@ -20,15 +20,27 @@ struct Batch {
 	int ninst;
 };
 
+// The boundary traces of a step's three stages (rk3_trace_block).
+template <typename T>
+struct Rk3Trace {
+	const double *bxyz; // [nbf][6][3]
+	long long nbf;
+	Batch b; // instances: data, dt, bfinst
+	const double *t_in; // [ninst] time
+	double *t_out; // [ninst] t_in + dt (advance)
+	T *out; // [3][nbf][6][6]
+	int advance; // 1: the traces of the next step
+};
+
 template <typename T>
 struct Rk3Params {
 	const T *w_in; // state read this stage, tiled (rk3_tix)
 	T *w_out; // state written this stage (ping-pong), tiled
 	T *k2; // low-storage register, in place, tiled
 	const T *geom; // codtau (row-major 3x3) and det, tiles of 32 elements x 10 values
-	const int *nb; // [ne][4] neighbour element, or -(boundary face + 1)
+	const int *nb; // [ne][4] neighbour element (all rows in the device order), or -(boundary face + 1)
 	const int *perm; // [ne][4] neighbour local node of face node jj, 4 bits each
-	const T *btrace; // [nbf][6][6] boundary data at t_stage (boundary_trace_kernel)
+	const T *btrace; // [nbf][6][6] boundary data at t_stage
 	const int *einst; // [ne] instance of each element, nullptr for one instance
 	const double *dt_tab; // [ninst] time step of each instance (used with einst)
 	long long ne;
@@ -39,6 +51,9 @@ struct Rk3Params {
 	int fact; // the derivative tables factor through the P1 basis (rk3_tables_factor)
 	int bc_metal; // boundary faces take the metal flux (-n x H_L, 0)
 	int num_sms; // SMs of the device
+	int traces; // the launch also writes tr (the last stage of a step)
+	int tile_blocks; // CTAs of the tiles, before those of tr (set at launch)
+	Rk3Trace<T> tr;
 	int idx32; // every tiled state offset fits 32 bits (ntiles * 1920 < 2^32)
 	int l2_ahead; // nonzero: prefetch into L2 the tile this many CTAs ahead (set per variant at launch)
 };
@@ -50,24 +65,30 @@ void rk3_sym_coeffs(const gdn_cuda_tables *t, double q4_sym[6], double minv_sym[
 bool rk3_tables_standard_faces(const gdn_cuda_tables *t);
 
 // variant 0 / 1: the stage kernel compiled for fewer / more resident CTAs per
-// SM (rk3_min_blocks), i.e. more / fewer registers per thread; FP32 with the P2
-// tables: rk3_elem_kernel (a thread per element), else rk3_stage_kernel
+// SM (rk3_min_blocks), i.e. more / fewer registers per thread.  With the P2
+// tables rk3_elem_kernel (FP32) or rk3_half_kernel (FP64), else rk3_stage_kernel
 template <typename T>
 int launch_rk3_stage(const Rk3Params<T> &p, int variant, cudaStream_t s);
 template <typename T>
 int prepare_rk3();
 
 int rk3_min_blocks(int precision_fp64, int fact, int variant);
-// reference layout [e][node][field] (FP64, elements 0..ne-1) <-> tiled layout
-// at elements e0 .. e0 + ne - 1
+// device element order: pos[e] (elements of one vertex-index stencil side by
+// side inside blocks, rk3_order_kernel), its inverse items[k], and the neighbour
+// / permutation rows in
+// that order (nb_out, perm_out [pos[e]][4])
+int launch_rk3_order(const int *e2q, const int *einst, const int *nb, const int *perm, long long ne, int *pos,
+					 int *items, int *nb_out, int *perm_out, cudaStream_t s);
+// reference layout [e][node][field] (FP64, ne elements) <-> tiled layout,
+// element e at position pos[e]
 template <typename T>
-int launch_rk3_to_tiles(const double *src, T *dst, long long e0, long long ne, cudaStream_t s);
+int launch_rk3_to_tiles(const double *src, T *dst, const int *pos, long long ne, cudaStream_t s);
 template <typename T>
-int launch_rk3_from_tiles(const T *src, double *dst, long long e0, long long ne, cudaStream_t s);
+int launch_rk3_from_tiles(const T *src, double *dst, const int *pos, long long ne, cudaStream_t s);
 template <typename T>
-int launch_geom_to_tiles(const double *g, T *out, long long ne, cudaStream_t s);
+int launch_geom_to_tiles(const double *g, T *out, const int *pos, long long ne, cudaStream_t s);
 template <typename T>
-int launch_boundary_trace(const double *bxyz, long long nbf, const Batch &b, double c_stage, T *out, cudaStream_t s);
+int launch_rk3_traces(const Rk3Trace<T> &tr, cudaStream_t s);
 int launch_set_time(const Batch &b, double value, cudaStream_t s);
 int launch_advance_time(const Batch &b, cudaStream_t s);
 
