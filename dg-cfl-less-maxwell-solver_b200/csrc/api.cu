@@ -58,6 +58,50 @@ extern "C" const char *gdn_cuda_last_error(void)
 			return _rc;                                                                            \
 	} while (0)
 
+// ------------------------------------------------------- device memory --
+namespace gdn {
+static std::mutex g_pool_mu;
+static std::map<int, cudaMemPool_t> g_pools; // by device, for the life of the process
+
+cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t s)
+{
+	int dev = 0;
+	cudaError_t e = cudaGetDevice(&dev);
+	if (e != cudaSuccess)
+		return e;
+	cudaMemPool_t pool = nullptr;
+	{
+		std::lock_guard<std::mutex> g(g_pool_mu);
+		auto it = g_pools.find(dev);
+		if (it != g_pools.end()) {
+			pool = it->second;
+		} else {
+			cudaMemPoolProps props = {};
+			props.allocType = cudaMemAllocationTypePinned;
+			props.location.type = cudaMemLocationTypeDevice;
+			props.location.id = dev;
+			e = cudaMemPoolCreate(&pool, &props);
+			if (e != cudaSuccess)
+				return e;
+			unsigned long long keep = kPoolKeep;
+			e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+			if (e != cudaSuccess) {
+				cudaMemPoolDestroy(pool);
+				return e;
+			}
+			g_pools[dev] = pool;
+		}
+	}
+	return cudaMallocFromPoolAsync(p, bytes, pool, s);
+}
+
+void dev_free(void *p, cudaStream_t s)
+{
+	if (p)
+		cudaFreeAsync(p, s);
+}
+} // namespace gdn
+
 // ---------------------------------------------------------------- handle --
 struct DevBuf {
 	void *p = nullptr;
@@ -166,7 +210,7 @@ static int dalloc(gdn_cuda_handle *h, X **p, size_t count)
 {
 	void *q = nullptr;
 	const size_t bytes = count * sizeof(X) > 0 ? count * sizeof(X) : 16;
-	cudaError_t e = cudaMalloc(&q, bytes);
+	cudaError_t e = dev_alloc(&q, bytes, h->stream);
 	if (e != cudaSuccess) {
 		cudaGetLastError();
 		char buf[160];
@@ -192,7 +236,9 @@ static void free_handle(gdn_cuda_handle *h)
 		if (h->graph_exec[k])
 			cudaGraphExecDestroy(h->graph_exec[k]);
 	for (auto &b : h->bufs)
-		cudaFree(b.p);
+		dev_free(b.p, h->stream);
+	if (h->stream)
+		cudaStreamSynchronize(h->stream); // what the pool does not keep goes back here
 	if (h->host_result)
 		cudaFreeHost(h->host_result);
 	if (h->stream)
@@ -476,6 +522,7 @@ static int autotune_rk3(gdn_cuda_handle *h)
 static int kin_prepare_grids(gdn_cuda_handle *h);
 static int kin_prepare_parts(gdn_cuda_handle *h, const gdn_cuda_mesh *m);
 static int autotune_kin(gdn_cuda_handle *h);
+static int kin_tuned_mode(gdn_cuda_handle *h, bool *timed);
 
 static int attach_impl(gdn_cuda_handle *h, const gdn_cuda_mesh *m, const gdn_cuda_tables *t,
 					   const gdn_cuda_model *mo)
@@ -679,9 +726,15 @@ static int attach_impl(gdn_cuda_handle *h, const gdn_cuda_mesh *m, const gdn_cud
 		GDN_CUDA_TRY(cudaMemcpyAsync(h->kgroups, groups.data(), groups.size() * sizeof(int2), cudaMemcpyHostToDevice,
 									 s));
 		GDN_TRY(kin_prepare_grids(h));
-		GDN_TRY(kin_prepare_parts(h, m));
 		GDN_CUDA_TRY(cudaStreamSynchronize(s));
+		// the spatial parts (host loops over the items) only where mode 4 runs or
+		// is timed
+		bool timed = false;
 		if (h->kin_autotune)
+			h->kin_mode = kin_tuned_mode(h, &timed);
+		if (h->kin_mode == 4 || (h->kin_autotune && !timed))
+			GDN_TRY(kin_prepare_parts(h, m));
+		if (h->kin_autotune && !timed)
 			GDN_TRY(autotune_kin(h));
 	}
 	return GDN_CUDA_OK;
@@ -1230,24 +1283,29 @@ static int kin_first_sweep(gdn_cuda_handle *h, long long &nl)
 // floor(log2 levels)) for the life of the process.
 static std::map<std::pair<int, int>, int> g_tune_kin;
 
-static int autotune_kin(gdn_cuda_handle *h)
+static std::pair<int, int> kin_tune_key(const gdn_cuda_handle *h)
 {
 	int ib = 0, lb = 0;
-	const long long nitems = h->ne * h->nv;
-	const long long nl = (long long)h->level_off.size() - 1;
-	while ((2LL << ib) <= nitems)
+	while ((2LL << ib) <= h->ne * h->nv)
 		ib++;
-	while ((2LL << lb) <= nl)
+	while ((2LL << lb) <= (long long)h->level_off.size() - 1)
 		lb++;
-	const std::pair<int, int> key(h->precision, ib * 64 + lb);
-	{
-		std::lock_guard<std::mutex> g(g_tune_mu);
-		auto it = g_tune_kin.find(key);
-		if (it != g_tune_kin.end()) {
-			h->kin_mode = it->second;
-			return GDN_CUDA_OK;
-		}
-	}
+	return std::pair<int, int>(h->precision, ib * 64 + lb);
+}
+
+// the mode timed before for this precision and size (*timed), or 1
+static int kin_tuned_mode(gdn_cuda_handle *h, bool *timed)
+{
+	std::lock_guard<std::mutex> g(g_tune_mu);
+	auto it = g_tune_kin.find(kin_tune_key(h));
+	*timed = it != g_tune_kin.end();
+	return *timed ? it->second : 1;
+}
+
+static int autotune_kin(gdn_cuda_handle *h)
+{
+	const long long nitems = h->ne * h->nv;
+	const std::pair<int, int> key = kin_tune_key(h);
 	GDN_CUDA_TRY(cudaMemsetAsync(h->f, 0, (size_t)60 * nitems * (h->precision == GDN_CUDA_FP32 ? 4 : h->precision == GDN_CUDA_BF16_STORE ? 2 : 8), h->stream));
 	GDN_CUDA_TRY(cudaMemsetAsync(h->bt, 0, (size_t)36 * h->nv * (h->nbf > 0 ? h->nbf : 1) * sizeof(double), h->stream));
 	// each mode: one warm-up solve, then the best of three solves timed one by

@@ -117,13 +117,13 @@ int kin_device_schedule(const unsigned char *mask, const int *nb, const double *
 	int rc = GDN_CUDA_OK;
 	int maxlev = 0;
 	auto cleanup = [&]() {
-		cudaFree(level);
-		cudaFree(lev_sorted);
-		cudaFree(iota);
-		cudaFree(indeg);
-		cudaFree(ctl);
-		cudaFree(loff);
-		cudaFree(tmp);
+		dev_free(level, s);
+		dev_free(lev_sorted, s);
+		dev_free(iota, s);
+		dev_free(indeg, s);
+		dev_free(ctl, s);
+		dev_free(loff, s);
+		dev_free(tmp, s);
 	};
 #define GDN_SCHED_TRY(expr)                                                                                           \
 	do {                                                                                                           \
@@ -133,11 +133,11 @@ int kin_device_schedule(const unsigned char *mask, const int *nb, const double *
 			return gdn_cuda_fail(_e, #expr, __FILE__, __LINE__);                                                  \
 		}                                                                                                          \
 	} while (0)
-	GDN_SCHED_TRY(cudaMalloc(&level, nu * sizeof(int)));
-	GDN_SCHED_TRY(cudaMalloc(&lev_sorted, nu * sizeof(int)));
-	GDN_SCHED_TRY(cudaMalloc(&iota, nu * sizeof(int)));
-	GDN_SCHED_TRY(cudaMalloc(&indeg, nu * sizeof(int)));
-	GDN_SCHED_TRY(cudaMalloc(&ctl, 8 * sizeof(unsigned)));
+	GDN_SCHED_TRY(dev_alloc(reinterpret_cast<void **>(&level), nu * sizeof(int), s));
+	GDN_SCHED_TRY(dev_alloc(reinterpret_cast<void **>(&lev_sorted), nu * sizeof(int), s));
+	GDN_SCHED_TRY(dev_alloc(reinterpret_cast<void **>(&iota), nu * sizeof(int), s));
+	GDN_SCHED_TRY(dev_alloc(reinterpret_cast<void **>(&indeg), nu * sizeof(int), s));
+	GDN_SCHED_TRY(dev_alloc(reinterpret_cast<void **>(&ctl), 8 * sizeof(unsigned), s));
 	GDN_SCHED_TRY(cudaMemsetAsync(ctl, 0, 8 * sizeof(unsigned), s));
 	// levels: Kahn's algorithm, the two frontiers in the sort buffers
 	{
@@ -166,21 +166,21 @@ int kin_device_schedule(const unsigned char *mask, const int *nb, const double *
 	{
 		int *dmax = reinterpret_cast<int *>(ctl + 7);
 		GDN_SCHED_TRY(cub::DeviceReduce::Max(nullptr, tmp_bytes, level, dmax, (int)nu, s));
-		GDN_SCHED_TRY(cudaMalloc(&tmp, tmp_bytes));
+		GDN_SCHED_TRY(dev_alloc(reinterpret_cast<void **>(&tmp), tmp_bytes, s));
 		GDN_SCHED_TRY(cub::DeviceReduce::Max(tmp, tmp_bytes, level, dmax, (int)nu, s));
 		GDN_SCHED_TRY(cudaMemcpyAsync(&maxlev, dmax, sizeof(int), cudaMemcpyDeviceToHost, s));
 		GDN_SCHED_TRY(cudaStreamSynchronize(s));
-		cudaFree(tmp);
+		dev_free(tmp, s);
 		tmp = nullptr;
 		while ((1 << bits) <= maxlev)
 			bits++;
 	}
 	GDN_SCHED_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, level, lev_sorted, iota, items, (int)nu, 0,
 												  bits, s));
-	GDN_SCHED_TRY(cudaMalloc(&tmp, tmp_bytes));
+	GDN_SCHED_TRY(dev_alloc(reinterpret_cast<void **>(&tmp), tmp_bytes, s));
 	GDN_SCHED_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, level, lev_sorted, iota, items, (int)nu, 0, bits,
 												  s));
-	GDN_SCHED_TRY(cudaMalloc(&loff, (maxlev + 2) * sizeof(int)));
+	GDN_SCHED_TRY(dev_alloc(reinterpret_cast<void **>(&loff), (maxlev + 2) * sizeof(int), s));
 	kin_schedule_finish_kernel<<<g, 256, 0, s>>>(items, lev_sorted, nu, pos, loff);
 	GDN_SCHED_TRY(cudaGetLastError());
 	level_off.assign(maxlev + 2, 0);
@@ -1219,15 +1219,15 @@ int kin_build_parts(const int *e2q, const double *node, long long ne, const doub
 	void *tmp = nullptr;
 	size_t tb = 0, tb2 = 0;
 	auto cleanup = [&]() {
-		cudaFree(code);
-		cudaFree(code_s);
-		cudaFree(elem);
-		cudaFree(elem_s);
-		cudaFree(pe);
-		cudaFree(pkey);
-		cudaFree(pkey_s);
-		cudaFree(iota);
-		cudaFree(tmp);
+		dev_free(code, s);
+		dev_free(code_s, s);
+		dev_free(elem, s);
+		dev_free(elem_s, s);
+		dev_free(pe, s);
+		dev_free(pkey, s);
+		dev_free(pkey_s, s);
+		dev_free(iota, s);
+		dev_free(tmp, s);
 	};
 #define GDN_PARTS_TRY(expr)                                                                                           \
 	do {                                                                                                           \
@@ -1237,14 +1237,14 @@ int kin_build_parts(const int *e2q, const double *node, long long ne, const doub
 			return gdn_cuda_fail(_e, #expr, __FILE__, __LINE__);                                                  \
 		}                                                                                                          \
 	} while (0)
-	GDN_PARTS_TRY(cudaMalloc(&code, ne * sizeof(unsigned)));
-	GDN_PARTS_TRY(cudaMalloc(&code_s, ne * sizeof(unsigned)));
-	GDN_PARTS_TRY(cudaMalloc(&elem, ne * sizeof(int)));
-	GDN_PARTS_TRY(cudaMalloc(&elem_s, ne * sizeof(int)));
-	GDN_PARTS_TRY(cudaMalloc(&pe, ne * sizeof(int)));
-	GDN_PARTS_TRY(cudaMalloc(&pkey, nitems * sizeof(int)));
-	GDN_PARTS_TRY(cudaMalloc(&pkey_s, nitems * sizeof(int)));
-	GDN_PARTS_TRY(cudaMalloc(&iota, nitems * sizeof(int)));
+	GDN_PARTS_TRY(dev_alloc(reinterpret_cast<void **>(&code), ne * sizeof(unsigned), s));
+	GDN_PARTS_TRY(dev_alloc(reinterpret_cast<void **>(&code_s), ne * sizeof(unsigned), s));
+	GDN_PARTS_TRY(dev_alloc(reinterpret_cast<void **>(&elem), ne * sizeof(int), s));
+	GDN_PARTS_TRY(dev_alloc(reinterpret_cast<void **>(&elem_s), ne * sizeof(int), s));
+	GDN_PARTS_TRY(dev_alloc(reinterpret_cast<void **>(&pe), ne * sizeof(int), s));
+	GDN_PARTS_TRY(dev_alloc(reinterpret_cast<void **>(&pkey), nitems * sizeof(int), s));
+	GDN_PARTS_TRY(dev_alloc(reinterpret_cast<void **>(&pkey_s), nitems * sizeof(int), s));
+	GDN_PARTS_TRY(dev_alloc(reinterpret_cast<void **>(&iota), nitems * sizeof(int), s));
 	double3 l = make_double3(lo[0], lo[1], lo[2]), ie;
 	ie.x = 1.0 / (hi[0] - lo[0] > 0.0 ? hi[0] - lo[0] : 1.0);
 	ie.y = 1.0 / (hi[1] - lo[1] > 0.0 ? hi[1] - lo[1] : 1.0);
@@ -1254,7 +1254,7 @@ int kin_build_parts(const int *e2q, const double *node, long long ne, const doub
 	GDN_PARTS_TRY(cudaGetLastError());
 	GDN_PARTS_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, code, code_s, elem, elem_s, (int)ne, 0, 30, s));
 	GDN_PARTS_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb2, pkey, pkey_s, iota, plist, (int)nitems, 0, 31, s));
-	GDN_PARTS_TRY(cudaMalloc(&tmp, tb > tb2 ? tb : tb2));
+	GDN_PARTS_TRY(dev_alloc(reinterpret_cast<void **>(&tmp), tb > tb2 ? tb : tb2, s));
 	tb = tb > tb2 ? tb : tb2;
 	GDN_PARTS_TRY(cub::DeviceRadixSort::SortPairs(tmp, tb, code, code_s, elem, elem_s, (int)ne, 0, 30, s));
 	kin_part_of_elem_kernel<<<ge, 256, 0, s>>>(elem_s, ne, nparts, pe);
