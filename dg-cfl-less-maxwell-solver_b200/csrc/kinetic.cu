@@ -577,9 +577,9 @@ __device__ __forceinline__ void store10(S *p, const T v[10])
 // G is read by its six lanes at one address (broadcast), one wavefront per
 // 16 bytes; a warp shares nothing with other warps, so there is no CTA barrier.
 // ms per step before (lane = item, 32 items per CTA) and after, the fastest
-// grouping of each (jittered meshes, d3q4): 17^3 FP64 0.76 / 0.45, 24^3 FP32 with
-// one refinement 3.03 / 1.47, 40^3 FP64 2.83 / 1.89, 64^3 FP32 5.83 / 3.62; a
-// level of 457 items takes 2.6 us (4.4 before), of 9250 items 3.5 us (7.4).
+// grouping of each (jittered meshes, d3q4): 17^3 FP64 0.76 / 0.43, 24^3 FP32 with
+// one refinement 3.03 / 1.38, 40^3 FP64 2.83 / 1.73, 64^3 FP32 5.83 / 3.62; a
+// level of 457 items takes 2.4 us (4.4 before), of 9250 items 3.5 us (7.4).
 constexpr int kSwSlots = 5; // items per warp
 
 // Warps per CTA (static shared memory below 48 KB) and items per CTA.
@@ -787,8 +787,11 @@ __device__ __forceinline__ void warp_gather(const KinSweepParams &p, const Sweep
 // Row-driven wait and gather: the rows are their own readiness flags.  Every
 // word of y is "unwritten" when the solve starts, and a trace is ready when it
 // is not: no flags, fences or ordering between an item's words are needed.
-// The rows are fetched at once; if a trace is missing, one lane per row polls
-// the row's last word, and the rows are fetched again when all have arrived.
+// One lane per row polls the row's last word until it is written; then the rows
+// are fetched, and polled on should a trace still be missing.  Most warps are
+// ahead of their inputs, so what waiting costs the others counts: lanes leave the
+// poll with their row, and no row is fetched in vain (fetching first and polling
+// all rows on: 40^3 FP64 1.83 against 1.73 ms per step, FP32 1.28 against 1.24).
 // false when *err is set, or after spin_limit polls (then *err is set here),
 // so a lost producer ends the launch instead of hanging it.
 template <typename F, typename T, int ACC>
@@ -798,7 +801,24 @@ __device__ __forceinline__ bool warp_gather_wait(const KinSweepParams &p, const 
 	const int mine = in.c == 0 ? nr[0] : (in.c == 1 ? nr[1] : (in.c == 2 ? nr[2] : -1));
 	const unsigned *last = reinterpret_cast<const unsigned *>(reinterpret_cast<const T *>(p.y) +
 															   (long long)(mine >= 0 ? mine : 0) * 60 + 60) - 1;
+	bool waiting = mine >= 0;
 	for (long long it = 0;; it++) {
+		for (;; it++) {
+			if (waiting) {
+				unsigned v;
+				asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(last) : "memory");
+				waiting = v == 0xffffffffu;
+			}
+			if (!__any_sync(0xffffffffu, waiting))
+				break;
+			if ((it & 63) == 63 && __any_sync(0xffffffffu, *(const volatile int *)err != 0))
+				return false;
+			if (it >= spin_limit) {
+				if ((threadIdx.x & 31) == 0)
+					atomicExch(err, 1);
+				return false;
+			}
+		}
 		warp_gather<F, T, ACC>(p, in, nr, sh, x);
 		bool missing = false;
 #pragma unroll
@@ -810,19 +830,10 @@ __device__ __forceinline__ bool warp_gather_wait(const KinSweepParams &p, const 
 			}
 		if (!__any_sync(0xffffffffu, missing))
 			return true;
-		for (;; it++) {
-			if ((it & 63) == 63 && __any_sync(0xffffffffu, *(const volatile int *)err != 0))
-				return false;
-			if (it >= spin_limit) {
-				if ((threadIdx.x & 31) == 0)
-					atomicExch(err, 1);
-				return false;
-			}
-			unsigned v = 0;
-			if (mine >= 0)
-				asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(last) : "memory");
-			if (!__any_sync(0xffffffffu, v == 0xffffffffu))
-				break;
+		if (it >= spin_limit) {
+			if ((threadIdx.x & 31) == 0)
+				atomicExch(err, 1);
+			return false;
 		}
 	}
 }
@@ -1134,8 +1145,10 @@ __global__ void __launch_bounds__(SweepCfg<T>::threads)
 // lowest level always has its inputs and a warp at work on it: the solve
 // progresses, and its critical path is the longest upwind chain, not the level
 // count times a launch.
+// Registers: 5 CTAs per SM fit at 96 (FP32) and 128 (FP64), 4 with an
+// accumulator (128).
 template <typename F, typename Y, typename T, int ACC, bool BD, bool SPARSE>
-__global__ void __launch_bounds__(SweepCfg<T>::threads)
+__global__ void __launch_bounds__(SweepCfg<T>::threads, sizeof(T) == 8 || ACC == 0 ? 5 : 4)
 	kin_flow_kernel(KinSweepParams p, const int2 *__restrict__ groups, int ngroups, const int *__restrict__ list,
 					const int *__restrict__ group_off, int *err, long long spin_limit)
 {
@@ -1147,6 +1160,26 @@ __global__ void __launch_bounds__(SweepCfg<T>::threads)
 		const int2 gr = groups[g];
 		long long k;
 		const int n = warp_items(gr.x, gr.y, k);
+		// the warp's next items into L2: block inverses, right-hand side, records
+		// (40^3 FP64 1.89 -> 1.85, 17^3 0.445 -> 0.432 ms per step)
+		if (!list && g + dg < g1) {
+			const int2 gn = groups[g + dg];
+			long long kn;
+			const int nn = warp_items(gn.x, gn.y, kn);
+			if (nn > 0) {
+				const int lane = threadIdx.x & 31;
+				if (lane == 0)
+					prefetch_l2(reinterpret_cast<const T *>(p.G) + kn * 100, nn * 100 * sizeof(T));
+				else if (lane == 1 && 60 * sizeof(F) % 16 == 0)
+					prefetch_l2(reinterpret_cast<const F *>(p.f) + kn * 60, nn * 60 * sizeof(F));
+				else if (lane == 2)
+					prefetch_l2(p.rnb + kn, nn * sizeof(int4));
+				else if (lane == 3)
+					prefetch_l2(p.rpm + kn, nn * sizeof(int4));
+				else if (lane == 4)
+					prefetch_l2(reinterpret_cast<const T *>(p.rs) + kn * 4, nn * 4 * sizeof(T));
+			}
+		}
 		if (n <= 0)
 			continue;
 		SweepLane<T, ACC> in;
@@ -1416,10 +1449,11 @@ int kin_flow_grid(int device, int acc, int sparse, int *grid)
 			 : acc == 1 ? (const void *)kin_flow_kernel<F, Y, T, 1, true, false>
 						: (const void *)kin_flow_kernel<F, Y, T, 2, false, false>;
 	GDN_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, SweepCfg<T>::threads, 0));
-	// at most 4 CTAs per SM: more warps in flight only poll (ms per step for 2, 3,
-	// 4 CTAs per SM and all that fit: 64^3 FP32 4.46, 3.93, 3.79, 3.80; 40^3 FP64
-	// 2.00, 1.93, 1.94, 1.94; 17^3 FP64 0.439, 0.443, 0.445, 0.450)
-	const int cap = 4;
+	// 16 to 20 warps per SM hold one to two levels of a large mesh; more only
+	// poll, fewer leave a level in parts (ms per step for 2, 3, 4, 5 CTAs per SM:
+	// 64^3 FP32 4.46, 3.93, 3.79, 3.62; 40^3 FP64 2.00, 1.93, 1.94, 1.94, before
+	// the polls below were thinned out)
+	const int cap = sizeof(T) == 4 ? 5 : 4;
 	*grid = nsm * (per > cap ? cap : (per > 0 ? per : 1));
 	return GDN_CUDA_OK;
 }
