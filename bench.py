@@ -328,8 +328,8 @@ def main():
                     help="profiling aid: comma-separated variants to run (rk3: fp64,fp32; kinetic: "
                          "fp64,fp32,fp32_refine1,fp32_refine2,bf16)")
     ap.add_argument("--kin-sweep", type=int, default=0, choices=[0, 1, 2, 3, 4],
-                    help="kinetic: force the sweep mode (1 level launches, 2 cooperative, 3 readiness "
-                         "flags, 4 spatial parts) and skip the per-mode timing; 0 = autotuned, with the "
+                    help="kinetic: force the sweep mode (1 level launches, 2 cooperative, 3 row-driven "
+                         "(its rows are its readiness flags), 4 spatial parts) and skip the per-mode timing; 0 = autotuned, with the "
                          "per-mode timing")
     ap.add_argument("--headline-only", action="store_true",
                     help="rk3: print the 96^3 line without the kinetic precision study and the batch")
