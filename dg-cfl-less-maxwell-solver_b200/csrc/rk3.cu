@@ -284,7 +284,9 @@ __device__ __forceinline__ void pdl_wait()
 // time and time step of the face's instance.  t is t_in, or with `advance` the next
 // step's time t_in + dt, which block 0 keeps in t_out (explicit.c:103).  Times are
 // formed with the host's rounding (no fused multiply-add), so every stage sees
-// the reference's time bits.
+// the reference's time bits.  A thread takes the three stages of a face node: the
+// trace CTAs have the stage kernel's footprint, so they are to be few (a stage
+// per thread: 96^3 FP32 2.39 against 2.33 ms per step).
 template <typename T>
 __device__ __forceinline__ void rk3_trace_block(const Rk3Trace<T> &tr, int blk)
 {
@@ -292,20 +294,23 @@ __device__ __forceinline__ void rk3_trace_block(const Rk3Trace<T> &tr, int blk)
 	if (blk == 0 && tr.advance)
 		for (int i = threadIdx.x; i < tr.b.ninst; i += blockDim.x)
 			tr.t_out[i] = __dadd_rn(tr.t_in[i], tr.b.dt[i]);
-	const long long u = blk * (long long)blockDim.x + threadIdx.x, per = tr.nbf * 6;
-	if (u >= 3 * per)
+	const long long q = blk * (long long)blockDim.x + threadIdx.x, per = tr.nbf * 6;
+	if (q >= per)
 		return;
-	const int stage = (int)(u / per);
-	const long long q = u - stage * per;
 	const int inst = tr.b.bfinst ? tr.b.bfinst[q / 6] : 0;
-	const double dt = tr.b.dt[inst], c = stage == 0 ? 0. : (stage == 1 ? 1. / 3. : 3. / 4.);
+	const double dt = tr.b.dt[inst];
 	const double t0 = tr.advance ? __dadd_rn(tr.t_in[inst], dt) : tr.t_in[inst];
 	const double x[3] = {tr.bxyz[3 * q], tr.bxyz[3 * q + 1], tr.bxyz[3 * q + 2]};
-	double we[6];
-	exact_w(tr.b.data[inst], x, __dadd_rn(t0, __dmul_rn(c, dt)), we);
+	const Data d = tr.b.data[inst];
 #pragma unroll
-	for (int k = 0; k < 6; k++)
-		tr.out[u * 6 + rk3_btrace_off<T>(k)] = (T)we[k];
+	for (int stage = 0; stage < 3; stage++) {
+		const double c = stage == 0 ? 0. : (stage == 1 ? 1. / 3. : 3. / 4.);
+		double we[6];
+		exact_w(d, x, __dadd_rn(t0, __dmul_rn(c, dt)), we);
+#pragma unroll
+		for (int k = 0; k < 6; k++)
+			tr.out[(stage * per + q) * 6 + rk3_btrace_off<T>(k)] = (T)we[k];
+	}
 }
 constexpr int kTraceThreads = 256;
 template <typename T>
@@ -316,7 +321,7 @@ __global__ void rk3_trace_kernel(Rk3Trace<T> tr)
 template <typename T>
 static int trace_blocks(const Rk3Trace<T> &tr, int threads)
 {
-	return (int)((tr.nbf * 18 + threads - 1) / threads) + (tr.nbf == 0);
+	return (int)((tr.nbf * 6 + threads - 1) / threads) + (tr.nbf == 0);
 }
 template <typename T>
 int launch_rk3_traces(const Rk3Trace<T> &tr, cudaStream_t s)
@@ -690,14 +695,14 @@ __global__ void __launch_bounds__(kRk3Threads, MINB) rk3_stage_kernel(Rk3Params<
 // of the layout make every step of the residual, which treats E and H alike,
 // packed FP32x2 arithmetic (the flux, the face mass, the derivatives, the lift
 // and the update): 64-bit rows instead of 32-bit ones, 2,250 instead of 6,670
-// warp instructions and 900 instead of 1,784 L1 wavefronts per tile and stage.
+// warp instructions and 720 instead of 1,784 L1 wavefronts per tile and stage.
 // The neighbour traces (72 pairs) are copied into the lane's own slots of shared
 // memory asynchronously, a group per face: they are in flight while the curl is
 // computed and hold no register.  k2 stays in registers (copying it too: 2.64 ms
 // per 96^3 step against 2.34).  It is bound by DRAM: 8 warps per SM at 188
 // registers reach 90 % of the copy bandwidth at 96^3; 12 warps at 168 registers
-// spill and reach 84 %.  ms per step, rk3_stage_kernel / this kernel: 27^3
-// 0.125 / 0.091, 48^3 0.556 / 0.328, 96^3 4.27 / 2.34.
+// spill and reach 84 %.  ms per step, rk3_stage_kernel at 7 launches / this kernel
+// at 3: 27^3 0.125 / 0.074, 48^3 0.556 / 0.306, 96^3 4.27 / 2.33.
 constexpr int kElemThreads = 128;
 struct Rk3Elem {
 	static constexpr int lo = 2, hi = 3; // CTAs per SM: 188 / 168 registers
