@@ -427,7 +427,9 @@ __device__ __forceinline__ void rk3_tile(const Rk3Params<T> &p, long long tile, 
 
 	int nbk[4] = {0, 0, 0, 0}, pmk[4] = {0, 0, 0, 0};
 	T cod[3][3], det = T(1);
-	// neighbour traces of this thread's flux slot (face node jj = warp) of face f
+	// neighbour traces of this thread's flux slot (face node jj = warp) of face f.
+	// Plain loads: the stage before may still be writing w_in and btrace when this
+	// grid starts, which the read-only path (__ldg) does not allow.
 	auto load_wR = [&](int f, T out[6]) {
 		const int nbv = nbk[f];
 		const int jj = warp;
@@ -436,12 +438,12 @@ __device__ __forceinline__ void rk3_tile(const Rk3Params<T> &p, long long tile, 
 			const T *g = p.w_in + rk3_tix<T>(nbv, qn * 6);
 #pragma unroll
 			for (int c = 0; c < 6; c++)
-				out[c] = __ldg(g + rk3_off<T>(0, c));
+				out[c] = g[rk3_off<T>(0, c)];
 		} else {
 			const T *g = p.btrace + ((long long)(-nbv - 1) * 6 + jj) * 6;
 #pragma unroll
 			for (int c = 0; c < 6; c++)
-				out[c] = __ldg(g + rk3_btrace_off<T>(c));
+				out[c] = g[rk3_btrace_off<T>(c)];
 		}
 	};
 	// Prefetched at the start so that the volume phase hides their latency:
