@@ -716,15 +716,16 @@ __device__ __forceinline__ void block_product<float>(const float *G, const float
 	}
 }
 
-// "Not written yet" in the solution array of the row-driven sweeps: all bits
-// set, a NaN that no arithmetic returns (for FP64 the upper word decides).
+// "Not written yet" in the solution array of the row-driven sweeps: all bits of
+// a value set, a NaN that no arithmetic returns by itself; written() keeps one
+// that was handed in (a payload of the state) out of the array.
 __device__ __forceinline__ bool unwritten(float v)
 {
 	return __float_as_uint(v) == 0xffffffffu;
 }
 __device__ __forceinline__ bool unwritten(double v)
 {
-	return (unsigned)__double2hiint(v) == 0xffffffffu;
+	return __double_as_longlong(v) == -1ll;
 }
 __device__ __forceinline__ float written(float v)
 {
@@ -732,7 +733,100 @@ __device__ __forceinline__ float written(float v)
 }
 __device__ __forceinline__ double written(double v)
 {
-	return unwritten(v) ? __hiloint2double(0x7fffffff, -1) : v;
+	return unwritten(v) ? __longlong_as_double(0x7fffffffffffffffll) : v;
+}
+
+// A lane's pieces of a row [6][10] that another CTA of the same launch writes or
+// reads: 16 bytes at 96 i bytes from p (lane c starts at 16 c), moved by relaxed
+// accesses of whole values.  A vector access counts as one access per element, so
+// the element type is the value's: a double is never seen in halves.
+template <typename T>
+struct RowPart;
+template <>
+struct RowPart<double> {
+	double2 v[5];
+	// on: else v stays as it is
+	__device__ __forceinline__ void load_relaxed(const double *p, int, bool on)
+	{
+		asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %11, 0;\n\t"
+					 "@q ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%10];\n\t"
+					 "@q ld.relaxed.gpu.global.v2.f64 {%2, %3}, [%10+96];\n\t"
+					 "@q ld.relaxed.gpu.global.v2.f64 {%4, %5}, [%10+192];\n\t"
+					 "@q ld.relaxed.gpu.global.v2.f64 {%6, %7}, [%10+288];\n\t"
+					 "@q ld.relaxed.gpu.global.v2.f64 {%8, %9}, [%10+384];\n\t}"
+					 : "+d"(v[0].x), "+d"(v[0].y), "+d"(v[1].x), "+d"(v[1].y), "+d"(v[2].x), "+d"(v[2].y),
+					   "+d"(v[3].x), "+d"(v[3].y), "+d"(v[4].x), "+d"(v[4].y)
+					 : "l"(p), "r"((int)on));
+	}
+	__device__ __forceinline__ void store_relaxed(double *p, int) const
+	{
+#pragma unroll
+		for (int i = 0; i < 5; i++)
+			asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p + 12 * i), "d"(v[i].x), "d"(v[i].y)
+						 : "memory");
+	}
+	__device__ __forceinline__ void load(const double *p, int)
+	{
+#pragma unroll
+		for (int i = 0; i < 5; i++)
+			v[i] = *reinterpret_cast<const double2 *>(p + 12 * i);
+	}
+	__device__ __forceinline__ void store(double *p, int) const
+	{
+#pragma unroll
+		for (int i = 0; i < 5; i++)
+			*reinterpret_cast<double2 *>(p + 12 * i) = v[i];
+	}
+};
+// 15 pieces: the third is that of lanes 0 to 2
+template <>
+struct RowPart<float> {
+	float4 v[3];
+	__device__ __forceinline__ void load_relaxed(const float *p, int c, bool on)
+	{
+		asm volatile("{\n\t.reg .pred q, r;\n\tsetp.ne.s32 q, %13, 0;\n\tsetp.ne.s32 r, %14, 0;\n\t"
+					 "@q ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%12];\n\t"
+					 "@q ld.relaxed.gpu.global.v4.f32 {%4, %5, %6, %7}, [%12+96];\n\t"
+					 "@r ld.relaxed.gpu.global.v4.f32 {%8, %9, %10, %11}, [%12+192];\n\t}"
+					 : "+f"(v[0].x), "+f"(v[0].y), "+f"(v[0].z), "+f"(v[0].w), "+f"(v[1].x), "+f"(v[1].y), "+f"(v[1].z),
+					   "+f"(v[1].w), "+f"(v[2].x), "+f"(v[2].y), "+f"(v[2].z), "+f"(v[2].w)
+					 : "l"(p), "r"((int)on), "r"((int)(on && c < 3)));
+	}
+	__device__ __forceinline__ void store_relaxed(float *p, int c) const
+	{
+#pragma unroll
+		for (int i = 0; i < 3; i++)
+			if (i < 2 || c < 3)
+				asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p + 24 * i), "f"(v[i].x),
+							 "f"(v[i].y), "f"(v[i].z), "f"(v[i].w)
+							 : "memory");
+	}
+	__device__ __forceinline__ void load(const float *p, int c)
+	{
+#pragma unroll
+		for (int i = 0; i < 3; i++)
+			if (i < 2 || c < 3)
+				v[i] = *reinterpret_cast<const float4 *>(p + 24 * i);
+	}
+	__device__ __forceinline__ void store(float *p, int c) const
+	{
+#pragma unroll
+		for (int i = 0; i < 3; i++)
+			if (i < 2 || c < 3)
+				*reinterpret_cast<float4 *>(p + 24 * i) = v[i];
+	}
+};
+__device__ __forceinline__ float load_relaxed(const float *p)
+{
+	float v;
+	asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+	return v;
+}
+__device__ __forceinline__ double load_relaxed(const double *p)
+{
+	double v;
+	asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+	return v;
 }
 
 // the neighbour item of the r-th inflow face (-1: none, or a boundary face)
@@ -752,42 +846,68 @@ __device__ __forceinline__ void inflow_rows(const SweepLane<T, ACC> &in, int nr[
 		}
 }
 
-// The inflow neighbours' whole rows into shared memory (through L2: L1 is not
+// The inflow neighbours' whole rows into shared memory through L2 (L1 is not
 // coherent with other SMs' writes made during the launch), then the lane's
-// traces x[f] (undefined on faces without inflow).  Call after warp_stage.
-template <typename F, typename T, int ACC>
+// traces x[f] (zero on faces without inflow).  Call after warp_stage.  FLOW:
+// the rows may be being written, so they are read by relaxed loads, all of them
+// in flight before the first goes to shared memory; else the rows are complete
+// and are copied asynchronously.
+template <typename F, typename T, int ACC, bool FLOW>
 __device__ __forceinline__ void warp_gather(const KinSweepParams &p, const SweepLane<T, ACC> &in, const int nr[3],
 											SweepWarp<F, T> &sh, T x[4][6])
 {
 	constexpr int YV = 16 / sizeof(T), YP = 60 / YV;
 	T *tr0 = sh.tr + in.slot * 180;
 	const T *y = reinterpret_cast<const T *>(p.y);
+	if (FLOW) {
+		// predicated loads on zeroed registers: branches (FP32 1.28 against 1.25 ms per
+		// 40^3 step), and registers that a skipped load leaves undefined stay alive
+		// around the loops and spill (1.71)
+		RowPart<T> v[3] = {};
 #pragma unroll
-	for (int r = 0; r < 3; r++)
-		if (nr[r] >= 0) {
-			const T *row = y + (long long)nr[r] * 60;
+		for (int r = 0; r < 3; r++)
+			v[r].load_relaxed(y + (long long)nr[r] * 60 + in.c * YV, in.c, nr[r] >= 0);
 #pragma unroll
-			for (int i = 0; i < (YP + 5) / 6; i++)
-				if (in.c + 6 * i < YP)
-					__pipeline_memcpy_async(tr0 + r * 60 + (in.c + 6 * i) * YV, row + (in.c + 6 * i) * YV, 16);
-		}
+		for (int r = 0; r < 3; r++)
+			if (nr[r] >= 0)
+				v[r].store(tr0 + r * 60 + in.c * YV, in.c);
+	} else {
+#pragma unroll
+		for (int r = 0; r < 3; r++)
+			if (nr[r] >= 0) {
+				const T *row = y + (long long)nr[r] * 60;
+#pragma unroll
+				for (int i = 0; i < (YP + 5) / 6; i++)
+					if (in.c + 6 * i < YP)
+						__pipeline_memcpy_async(tr0 + r * 60 + (in.c + 6 * i) * YV, row + (in.c + 6 * i) * YV, 16);
+			}
+	}
 	__pipeline_commit();
 	__pipeline_wait_prior(0);
 	__syncwarp();
 #pragma unroll
-	for (int f = 0; f < 4; f++)
+	for (int f = 0; f < 4; f++) {
+#pragma unroll
+		for (int jj = 0; jj < 6; jj++)
+			x[f][jj] = T(0); // not a value of an earlier fetch: x is dead while the rows are waited for
 		if (in.inflow >> f & 1) {
 			const T *row = tr0 + __popc(in.inflow & ((1u << f) - 1)) * 60 + in.c * 10;
 #pragma unroll
 			for (int jj = 0; jj < 6; jj++)
 				x[f][jj] = row[(in.pmk[f] >> (4 * jj)) & 15];
 		}
+	}
 }
 
 // Row-driven wait and gather: the rows are their own readiness flags.  Every
-// word of y is "unwritten" when the solve starts, and a trace is ready when it
-// is not: no flags, fences or ordering between an item's words are needed.
-// One lane per row polls the row's last word until it is written; then the rows
+// value of y is "unwritten" when the solve starts and is written once, whole, by
+// a relaxed store of its size; every trace is read by a relaxed load of that size
+// and is ready when it is not "unwritten".  Nothing else passes between the CTAs,
+// so no flag, fence or ordering between the values of a row is needed.  (Rows copied
+// by cp.async are not atomic by the memory model; ms per step with them / as here:
+// 17^3 FP64 0.428 / 0.457, 40^3 FP64 1.73 / 1.82, 40^3 FP32 1.23 / 1.25, 64^3 FP32
+// 3.64 / 3.66.  A fence and a flag per warp: 17^3 0.67, 64^3 4.4.)
+// One lane per row polls the row's last value until it is written; then the rows
 // are fetched, and polled on should a trace still be missing.  Most warps are
 // ahead of their inputs, so what waiting costs the others counts: lanes leave the
 // poll with their row, and no row is fetched in vain (fetching first and polling
@@ -799,16 +919,12 @@ __device__ __forceinline__ bool warp_gather_wait(const KinSweepParams &p, const 
 												 SweepWarp<F, T> &sh, T x[4][6], int *err, long long spin_limit)
 {
 	const int mine = in.c == 0 ? nr[0] : (in.c == 1 ? nr[1] : (in.c == 2 ? nr[2] : -1));
-	const unsigned *last = reinterpret_cast<const unsigned *>(reinterpret_cast<const T *>(p.y) +
-															   (long long)(mine >= 0 ? mine : 0) * 60 + 60) - 1;
+	const T *last = reinterpret_cast<const T *>(p.y) + (long long)(mine >= 0 ? mine : 0) * 60 + 59;
 	bool waiting = mine >= 0;
 	for (long long it = 0;; it++) {
 		for (;; it++) {
-			if (waiting) {
-				unsigned v;
-				asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(last) : "memory");
-				waiting = v == 0xffffffffu;
-			}
+			if (waiting)
+				waiting = unwritten(load_relaxed(last));
 			if (!__any_sync(0xffffffffu, waiting))
 				break;
 			if ((it & 63) == 63 && __any_sync(0xffffffffu, *(const volatile int *)err != 0))
@@ -819,7 +935,7 @@ __device__ __forceinline__ bool warp_gather_wait(const KinSweepParams &p, const 
 				return false;
 			}
 		}
-		warp_gather<F, T, ACC>(p, in, nr, sh, x);
+		warp_gather<F, T, ACC, true>(p, in, nr, sh, x);
 		bool missing = false;
 #pragma unroll
 		for (int f = 0; f < 4; f++)
@@ -846,7 +962,7 @@ template <typename F, typename T, int ACC, bool SPARSE, bool FLOW>
 __device__ __forceinline__ void warp_solve(const KinSweepParams &p, const SweepLane<T, ACC> &in, const T x[4][6],
 										   SweepWarp<F, T> &sh)
 {
-	constexpr int YV = 16 / sizeof(T), YP = 60 / YV;
+	constexpr int YV = 16 / sizeof(T);
 	const Tables<T> &tb = tab<T>();
 	const int slot = in.slot, c = in.c;
 	T *tr0 = sh.tr + slot * 180;
@@ -888,12 +1004,13 @@ __device__ __forceinline__ void warp_solve(const KinSweepParams &p, const SweepL
 		store10<T, T>(tr0 + c * 10, y);
 	__syncwarp();
 	if (in.act) {
-		T *yo = reinterpret_cast<T *>(p.y) + in.k * 60;
-#pragma unroll
-		for (int i = 0; i < (YP + 5) / 6; i++)
-			if (c + 6 * i < YP)
-				*reinterpret_cast<float4 *>(yo + (c + 6 * i) * YV) =
-					*reinterpret_cast<const float4 *>(tr0 + (c + 6 * i) * YV);
+		T *yo = reinterpret_cast<T *>(p.y) + in.k * 60 + c * YV;
+		RowPart<T> v;
+		v.load(tr0 + c * YV, c);
+		if (FLOW)
+			v.store_relaxed(yo, c);
+		else
+			v.store(yo, c);
 		if (ACC != 0) {
 			double2 *ya = reinterpret_cast<double2 *>(p.yacc + in.k * 60);
 #pragma unroll
@@ -934,7 +1051,7 @@ __global__ void __launch_bounds__(SweepCfg<T>::threads) kin_sweep_kernel(KinSwee
 	T x[4][6];
 	inflow_rows(in, nr);
 	asm volatile("griddepcontrol.wait;" ::: "memory");
-	warp_gather<F, T, ACC>(p, in, nr, sh[threadIdx.x >> 5], x);
+	warp_gather<F, T, ACC, false>(p, in, nr, sh[threadIdx.x >> 5], x);
 	warp_solve<F, T, ACC, SPARSE, false>(p, in, x, sh[threadIdx.x >> 5]);
 }
 
@@ -1124,7 +1241,7 @@ __global__ void __launch_bounds__(SweepCfg<T>::threads)
 				int nr[3];
 				T x[4][6];
 				inflow_rows(in, nr);
-				warp_gather<F, T, ACC>(p, in, nr, sh[threadIdx.x >> 5], x);
+				warp_gather<F, T, ACC, false>(p, in, nr, sh[threadIdx.x >> 5], x);
 				warp_solve<F, T, ACC, SPARSE, false>(p, in, x, sh[threadIdx.x >> 5]);
 			}
 		}
