@@ -939,7 +939,7 @@ __device__ __forceinline__ bool warp_gather_wait(const KinSweepParams &p, const 
 		bool missing = false;
 #pragma unroll
 		for (int f = 0; f < 4; f++)
-			if (in.inflow >> f & 1) {
+			if ((in.inflow >> f & 1) && in.nbk[f] >= 0) { // boundary values carry no mark
 #pragma unroll
 				for (int jj = 0; jj < 6; jj++)
 					missing |= unwritten(x[f][jj]);

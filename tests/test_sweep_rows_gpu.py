@@ -38,3 +38,23 @@ def test_odd_values_pass_through_every_mode(n, nb_v, precision):
             first = got
             assert np.isnan(got).any() and np.isfinite(got).any()
         assert np.array_equal(got, first, equal_nan=True), mode
+
+
+@pytest.mark.parametrize("precision", [capi.FP64, capi.FP32, capi.FP32_REFINE, capi.BF16_STORE])
+@pytest.mark.parametrize("data", [capi.plane_data(), capi.cavity_data()])
+def test_boundary_data_may_be_the_mark_itself(precision, data):
+    """A time that is the NaN pattern makes boundary values that are; nothing may
+    wait for them to be written."""
+    c, e = kuhn.kuhn_cube(2, 0.1, seed=1)
+    mesh = capi.mesh_build(c, e)
+    t = np.array([BITS[0]], np.uint64).view(np.float64)[0]
+    first = None
+    for mode in (1, 2, 3, 4):
+        s = capi.Solver(mesh, capi.SCHEME_KINETIC, data, 6 * mesh.hmin(), precision=precision, kin_sweep=mode)
+        s.set_wait_limit(1 << 18)
+        s.set_state(np.random.default_rng(1).standard_normal(s.wlen), t)
+        s.advance(1)
+        got = s.get_state()
+        s.close()
+        first = got if first is None else first
+        assert np.array_equal(got, first, equal_nan=True), mode
