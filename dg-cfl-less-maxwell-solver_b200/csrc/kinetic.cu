@@ -1035,7 +1035,8 @@ __device__ __forceinline__ int warp_items(long long k0, long long k1, long long 
 
 // One level per launch, with programmatic dependent launch: the next level's
 // CTAs stage their items (data no sweep level writes) while this level runs,
-// and wait (griddepcontrol.wait) only before they read the upwind rows.
+// and wait (griddepcontrol.wait) only before they read the upwind rows.  The first
+// level is an ordinary launch (launch_kin_sweep).
 template <typename F, typename Y, typename T, int ACC, bool BD, bool SPARSE>
 __global__ void __launch_bounds__(SweepCfg<T>::threads) kin_sweep_kernel(KinSweepParams p)
 {
@@ -1441,7 +1442,10 @@ int launch_kin_sweep(const KinSweepParams &p, int acc, int bdata, int sparse, cu
 	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
 	attr[0].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = attr;
-	cfg.numAttrs = 1;
+	// The first level stages what the kernels just before it wrote (boundary data,
+	// right-hand side), ahead of griddepcontrol.wait: it is an ordinary launch, which
+	// starts after them.  A later level starts after the first has.
+	cfg.numAttrs = p.item_begin > 0 ? 1 : 0;
 #define GDN_SWEEP(A, B, SP) GDN_CUDA_TRY(cudaLaunchKernelEx(&cfg, kin_sweep_kernel<F, Y, T, A, B, SP>, p))
 	if (acc == 0 && bdata) {
 		if (sparse)

@@ -49,3 +49,13 @@ def test_waiting_and_gathering_use_them():
     flow = _body(_body(src, r"void warp_gather\("), r"if \(FLOW\)")
     assert "load_relaxed" in flow and "memcpy_async" not in flow
     assert re.search(r"if \(FLOW\)\s*v\.store_relaxed", _body(src, r"void warp_solve\("))
+
+
+def test_the_first_level_is_an_ordinary_launch():
+    """Levels stage right-hand side and boundary data ahead of their grid dependency
+    wait.  The first one's are written by the kernels just before it, so it must not
+    start early; the later ones' are then complete."""
+    body = _body(_source(), r"int launch_kin_sweep\(")
+    assert re.search(r"numAttrs = p\.item_begin > 0 \? 1 : 0;", body)
+    stage = _body(_source(), r"void warp_stage\(")
+    assert "p.bt" in stage and "p.yacc" in stage  # still staged ahead
