@@ -570,10 +570,13 @@ __device__ __forceinline__ void store10(S *p, const T v[10])
 //   stage   G and f of the item into shared memory (cp.async), its records
 //           into registers (data no sweep step writes);
 //   wait    the caller waits for the item's upwind neighbours;
-//   solve   the whole row of each inflow neighbour (at most three faces: sum s
-//           = 0) into shared memory through L2, one round trip; the face
-//           permutation then picks the traces out of the row there; y leaves
-//           through shared memory in the same 16-byte pieces.
+//   solve   the whole row of each inflow neighbour (three at most) into shared
+//           memory through L2, one round trip; the face permutation then picks
+//           the traces out of the row there; y leaves through shared memory in
+//           the same 16-byte pieces.
+// An item has at most three inflow faces where the two sides of a face agree (sum
+// s = 0).  The attach takes meshes whose sides differ, and there it can have four:
+// the traces of face 3 are then read one by one (all_inflow).
 // G is read by its six lanes at one address (broadcast), one wavefront per
 // 16 bytes; a warp shares nothing with other warps, so there is no CTA barrier.
 // ms per step before (lane = item, 32 items per CTA) and after, the fastest
@@ -613,6 +616,13 @@ struct SweepLane {
 	T s[4], coef;
 	double2 ya[ACC == 2 ? 5 : 1];
 };
+
+// the item has four inflow faces: face 3 has no place among the three rows
+template <typename T, int ACC>
+__device__ __forceinline__ bool all_inflow(const SweepLane<T, ACC> &in)
+{
+	return in.inflow == 15u;
+}
 
 // nloc (1 to 5) items k0 .. k0 + nloc - 1, or with `list` list[k0 ..].
 template <typename F, typename T, int ACC, bool BD>
@@ -667,7 +677,7 @@ __device__ __forceinline__ void warp_stage(const KinSweepParams &p, long long k0
 	if (BD) { // boundary inflow faces: f_eq of the data, in face order
 #pragma unroll
 		for (int f = 0; f < 4; f++)
-			if ((in.inflow >> f & 1) && in.nbk[f] < 0) {
+			if ((in.inflow >> f & 1) && in.nbk[f] < 0 && !(f == 3 && all_inflow(in))) {
 				const int r = __popc(in.inflow & ((1u << f) - 1));
 				const int v = p.items[k] % p.nv;
 				const double *b = p.bt + (((long long)(-in.nbk[f] - 1) * p.nv + v) * 6 + c) * 6;
@@ -846,13 +856,24 @@ __device__ __forceinline__ void inflow_rows(const SweepLane<T, ACC> &in, int nr[
 		}
 }
 
+// trace jj of face 3 of an item with four inflow faces, from where it is
+template <typename F, typename T, int ACC, bool BD>
+__device__ __forceinline__ T last_trace(const KinSweepParams &p, const SweepLane<T, ACC> &in, int jj)
+{
+	if (in.nbk[3] >= 0)
+		return load_relaxed(reinterpret_cast<const T *>(p.y) + (long long)in.nbk[3] * 60 + in.c * 10 +
+							((in.pmk[3] >> (4 * jj)) & 15));
+	const int v = p.items[in.k] % p.nv;
+	return BD ? (T)p.bt[(((long long)(-in.nbk[3] - 1) * p.nv + v) * 6 + in.c) * 6 + jj] : T(0);
+}
+
 // The inflow neighbours' whole rows into shared memory through L2 (L1 is not
 // coherent with other SMs' writes made during the launch), then the lane's
 // traces x[f] (zero on faces without inflow).  Call after warp_stage.  FLOW:
 // the rows may be being written, so they are read by relaxed loads, all of them
 // in flight before the first goes to shared memory; else the rows are complete
 // and are copied asynchronously.
-template <typename F, typename T, int ACC, bool FLOW>
+template <typename F, typename T, int ACC, bool BD, bool FLOW>
 __device__ __forceinline__ void warp_gather(const KinSweepParams &p, const SweepLane<T, ACC> &in, const int nr[3],
 											SweepWarp<F, T> &sh, T x[4][6])
 {
@@ -891,6 +912,19 @@ __device__ __forceinline__ void warp_gather(const KinSweepParams &p, const Sweep
 		for (int jj = 0; jj < 6; jj++)
 			x[f][jj] = T(0); // not a value of an earlier fetch: x is dead while the rows are waited for
 		if (in.inflow >> f & 1) {
+			if (f == 3 && all_inflow(in)) {
+#pragma unroll 1
+				for (int jj = 0; jj < 6; jj++) {
+					const T v = last_trace<F, T, ACC, BD>(p, in, jj);
+					x[3][0] = jj == 0 ? v : x[3][0];
+					x[3][1] = jj == 1 ? v : x[3][1];
+					x[3][2] = jj == 2 ? v : x[3][2];
+					x[3][3] = jj == 3 ? v : x[3][3];
+					x[3][4] = jj == 4 ? v : x[3][4];
+					x[3][5] = jj == 5 ? v : x[3][5];
+				}
+				continue;
+			}
 			const T *row = tr0 + __popc(in.inflow & ((1u << f) - 1)) * 60 + in.c * 10;
 #pragma unroll
 			for (int jj = 0; jj < 6; jj++)
@@ -914,11 +948,11 @@ __device__ __forceinline__ void warp_gather(const KinSweepParams &p, const Sweep
 // all rows on: 40^3 FP64 1.83 against 1.73 ms per step, FP32 1.28 against 1.24).
 // false when *err is set, or after spin_limit polls (then *err is set here),
 // so a lost producer ends the launch instead of hanging it.
-template <typename F, typename T, int ACC>
+template <typename F, typename T, int ACC, bool BD>
 __device__ __forceinline__ bool warp_gather_wait(const KinSweepParams &p, const SweepLane<T, ACC> &in, const int nr[3],
 												 SweepWarp<F, T> &sh, T x[4][6], int *err, long long spin_limit)
 {
-	const int mine = in.c == 0 ? nr[0] : (in.c == 1 ? nr[1] : (in.c == 2 ? nr[2] : -1));
+	const int mine = in.c == 0 ? nr[0] : (in.c == 1 ? nr[1] : (in.c == 2 ? nr[2] : (in.c == 3 && all_inflow(in) ? in.nbk[3] : -1)));
 	const T *last = reinterpret_cast<const T *>(p.y) + (long long)(mine >= 0 ? mine : 0) * 60 + 59;
 	bool waiting = mine >= 0;
 	for (long long it = 0;; it++) {
@@ -935,7 +969,7 @@ __device__ __forceinline__ bool warp_gather_wait(const KinSweepParams &p, const 
 				return false;
 			}
 		}
-		warp_gather<F, T, ACC, true>(p, in, nr, sh, x);
+		warp_gather<F, T, ACC, BD, true>(p, in, nr, sh, x);
 		bool missing = false;
 #pragma unroll
 		for (int f = 0; f < 4; f++)
@@ -1052,7 +1086,7 @@ __global__ void __launch_bounds__(SweepCfg<T>::threads) kin_sweep_kernel(KinSwee
 	T x[4][6];
 	inflow_rows(in, nr);
 	asm volatile("griddepcontrol.wait;" ::: "memory");
-	warp_gather<F, T, ACC, false>(p, in, nr, sh[threadIdx.x >> 5], x);
+	warp_gather<F, T, ACC, BD, false>(p, in, nr, sh[threadIdx.x >> 5], x);
 	warp_solve<F, T, ACC, SPARSE, false>(p, in, x, sh[threadIdx.x >> 5]);
 }
 
@@ -1242,7 +1276,7 @@ __global__ void __launch_bounds__(SweepCfg<T>::threads)
 				int nr[3];
 				T x[4][6];
 				inflow_rows(in, nr);
-				warp_gather<F, T, ACC, false>(p, in, nr, sh[threadIdx.x >> 5], x);
+				warp_gather<F, T, ACC, BD, false>(p, in, nr, sh[threadIdx.x >> 5], x);
 				warp_solve<F, T, ACC, SPARSE, false>(p, in, x, sh[threadIdx.x >> 5]);
 			}
 		}
@@ -1305,7 +1339,7 @@ __global__ void __launch_bounds__(SweepCfg<T>::threads, sizeof(T) == 8 || ACC ==
 		int nr[3];
 		T x[4][6];
 		inflow_rows(in, nr);
-		if (!warp_gather_wait<F, T, ACC>(p, in, nr, sh[threadIdx.x >> 5], x, err, spin_limit))
+		if (!warp_gather_wait<F, T, ACC, BD>(p, in, nr, sh[threadIdx.x >> 5], x, err, spin_limit))
 			return; // *err is set; the state of this solve is invalid
 		warp_solve<F, T, ACC, SPARSE, true>(p, in, x, sh[threadIdx.x >> 5]);
 	}

@@ -45,7 +45,7 @@ def test_waiting_and_gathering_use_them():
     src = _source()
     wait = _body(src, r"bool warp_gather_wait\(")
     assert "unwritten(load_relaxed(last))" in wait and ".u32" not in wait
-    assert re.search(r"warp_gather<F, T, ACC, true>", wait)
+    assert re.search(r"warp_gather<F, T, ACC, (BD, )?true>", wait)
     flow = _body(_body(src, r"void warp_gather\("), r"if \(FLOW\)")
     assert "load_relaxed" in flow and "memcpy_async" not in flow
     assert re.search(r"if \(FLOW\)\s*v\.store_relaxed", _body(src, r"void warp_solve\("))
