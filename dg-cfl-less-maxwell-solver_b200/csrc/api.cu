@@ -7,6 +7,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <utility>
 #include <vector>
@@ -60,8 +61,30 @@ extern "C" const char *gdn_cuda_last_error(void)
 
 // ------------------------------------------------------- device memory --
 namespace gdn {
-static std::mutex g_pool_mu;
-static std::map<int, cudaMemPool_t> g_pools; // by device, for the life of the process
+struct DevMem {
+	cudaMemPool_t pool = nullptr; // for the life of the process
+	std::set<void *> plain; // blocks of cudaMalloc
+};
+static std::mutex g_mem_mu;
+static std::map<int, DevMem> g_mem; // by device
+
+static cudaError_t make_pool(int dev, cudaMemPool_t *pool)
+{
+	cudaMemPoolProps props = {};
+	props.allocType = cudaMemAllocationTypePinned;
+	props.location.type = cudaMemLocationTypeDevice;
+	props.location.id = dev;
+	cudaError_t e = cudaMemPoolCreate(pool, &props);
+	if (e != cudaSuccess)
+		return e;
+	unsigned long long keep = kPoolKeep;
+	e = cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep);
+	if (e != cudaSuccess) {
+		cudaMemPoolDestroy(*pool);
+		*pool = nullptr;
+	}
+	return e;
+}
 
 cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t s)
 {
@@ -69,35 +92,41 @@ cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t s)
 	cudaError_t e = cudaGetDevice(&dev);
 	if (e != cudaSuccess)
 		return e;
+	if (bytes > kPoolBlock) {
+		e = cudaMalloc(p, bytes);
+		if (e == cudaSuccess) {
+			std::lock_guard<std::mutex> g(g_mem_mu);
+			g_mem[dev].plain.insert(*p);
+		}
+		return e;
+	}
 	cudaMemPool_t pool = nullptr;
 	{
-		std::lock_guard<std::mutex> g(g_pool_mu);
-		auto it = g_pools.find(dev);
-		if (it != g_pools.end()) {
-			pool = it->second;
-		} else {
-			cudaMemPoolProps props = {};
-			props.allocType = cudaMemAllocationTypePinned;
-			props.location.type = cudaMemLocationTypeDevice;
-			props.location.id = dev;
-			e = cudaMemPoolCreate(&pool, &props);
+		std::lock_guard<std::mutex> g(g_mem_mu);
+		DevMem &m = g_mem[dev];
+		if (!m.pool) {
+			e = make_pool(dev, &m.pool);
 			if (e != cudaSuccess)
 				return e;
-			unsigned long long keep = kPoolKeep;
-			e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-			if (e != cudaSuccess) {
-				cudaMemPoolDestroy(pool);
-				return e;
-			}
-			g_pools[dev] = pool;
 		}
+		pool = m.pool;
 	}
 	return cudaMallocFromPoolAsync(p, bytes, pool, s);
 }
 
 void dev_free(void *p, cudaStream_t s)
 {
-	if (p)
+	int dev = 0;
+	if (!p || cudaGetDevice(&dev) != cudaSuccess)
+		return;
+	bool plain;
+	{
+		std::lock_guard<std::mutex> g(g_mem_mu);
+		plain = g_mem[dev].plain.erase(p) > 0;
+	}
+	if (plain)
+		cudaFree(p); // waits for the device, as what may still read the block is on it
+	else
 		cudaFreeAsync(p, s);
 }
 } // namespace gdn
