@@ -62,11 +62,50 @@ extern "C" const char *gdn_cuda_last_error(void)
 // ------------------------------------------------------- device memory --
 namespace gdn {
 struct DevMem {
-	cudaMemPool_t pool = nullptr; // for the life of the process
+	unsigned long long ctx = 0; // the context the rest belongs to
+	cudaMemPool_t pool = nullptr; // for the life of the context
 	std::set<void *> plain; // blocks of cudaMalloc
 };
 static std::mutex g_mem_mu;
 static std::map<int, DevMem> g_mem; // by device
+
+// The current context's number: a host that resets the device (cudaDeviceReset) gets
+// a new one, and the pool and blocks of the old one are gone with it.
+static cudaError_t context_id(unsigned long long *id)
+{
+	typedef int (*get_id_t)(void *ctx, unsigned long long *id); // cuCtxGetId
+	static get_id_t fn = nullptr;
+	static std::once_flag once;
+	std::call_once(once, [] {
+		void *f = nullptr;
+		cudaDriverEntryPointQueryResult q;
+		if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+			q == cudaDriverEntryPointSuccess)
+			fn = reinterpret_cast<get_id_t>(f);
+	});
+	if (!fn)
+		return cudaErrorNotSupported;
+	cudaError_t e = cudaFree(nullptr); // makes the primary context current
+	if (e != cudaSuccess)
+		return e;
+	return fn(nullptr, id) == 0 ? cudaSuccess : cudaErrorDeviceUninitialized;
+}
+
+// the entry of the current device and context (g_mem_mu is held)
+static cudaError_t mem_of(int dev, DevMem **out)
+{
+	unsigned long long id = 0;
+	cudaError_t e = context_id(&id);
+	if (e != cudaSuccess)
+		return e;
+	DevMem &m = g_mem[dev];
+	if (m.ctx != id) {
+		m = DevMem();
+		m.ctx = id;
+	}
+	*out = &m;
+	return cudaSuccess;
+}
 
 static cudaError_t make_pool(int dev, cudaMemPool_t *pool)
 {
@@ -92,24 +131,28 @@ cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t s)
 	cudaError_t e = cudaGetDevice(&dev);
 	if (e != cudaSuccess)
 		return e;
+	DevMem *m = nullptr;
 	if (bytes > kPoolBlock) {
 		e = cudaMalloc(p, bytes);
-		if (e == cudaSuccess) {
-			std::lock_guard<std::mutex> g(g_mem_mu);
-			g_mem[dev].plain.insert(*p);
-		}
+		if (e != cudaSuccess)
+			return e;
+		std::lock_guard<std::mutex> g(g_mem_mu);
+		e = mem_of(dev, &m);
+		if (e == cudaSuccess)
+			m->plain.insert(*p);
+		else
+			cudaFree(*p);
 		return e;
 	}
 	cudaMemPool_t pool = nullptr;
 	{
 		std::lock_guard<std::mutex> g(g_mem_mu);
-		DevMem &m = g_mem[dev];
-		if (!m.pool) {
-			e = make_pool(dev, &m.pool);
-			if (e != cudaSuccess)
-				return e;
-		}
-		pool = m.pool;
+		e = mem_of(dev, &m);
+		if (e == cudaSuccess && !m->pool)
+			e = make_pool(dev, &m->pool);
+		if (e != cudaSuccess)
+			return e;
+		pool = m->pool;
 	}
 	return cudaMallocFromPoolAsync(p, bytes, pool, s);
 }
@@ -119,10 +162,12 @@ void dev_free(void *p, cudaStream_t s)
 	int dev = 0;
 	if (!p || cudaGetDevice(&dev) != cudaSuccess)
 		return;
-	bool plain;
+	bool plain = false;
 	{
 		std::lock_guard<std::mutex> g(g_mem_mu);
-		plain = g_mem[dev].plain.erase(p) > 0;
+		DevMem *m = nullptr;
+		if (mem_of(dev, &m) == cudaSuccess)
+			plain = m->plain.erase(p) > 0;
 	}
 	if (plain)
 		cudaFree(p); // waits for the device, as what may still read the block is on it
