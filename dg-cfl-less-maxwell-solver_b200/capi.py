@@ -80,7 +80,7 @@ EXPORTS = [
     "gdn_cuda_error_l2_batch", "gdn_cuda_num_instances", "gdn_cuda_instance_info", "gdn_cuda_rk3_variant",
     "gdn_cuda_kin_sweep_mode", "gdn_cuda_time_convergence", "gdn_cuda_space_convergence",
     "gdn_cuda_mesh_build_gpu", "gdn_cuda_save_xdmf", "gdn_cuda_eval_data",
-    "gdn_cuda_set_wait_limit",
+    "gdn_cuda_set_wait_limit", "gdn_cuda_release_memory",
 ]
 
 _lib = None
@@ -103,6 +103,7 @@ def lib():
     L.gdn_cuda_attach.argtypes = [C.POINTER(Mesh), C.POINTER(Tables), C.POINTER(Model),
                                   C.POINTER(Data), C.POINTER(Config), C.c_double, C.POINTER(vp)]
     L.gdn_cuda_detach.argtypes = [vp]
+    L.gdn_cuda_release_memory.argtypes = [C.c_int]
     L.gdn_cuda_solve.argtypes = [vp, C.c_int, dp, dp, dp]
     L.gdn_cuda_init.argtypes = [vp]
     L.gdn_cuda_advance.argtypes = [vp, C.c_int]
@@ -147,6 +148,11 @@ def _ip(a):
 
 def _dp(a):
     return a.ctypes.data_as(C.POINTER(C.c_double))
+
+
+def release_memory(device: int = 0):
+    """Gives the device memory that the library keeps between handles back."""
+    check(lib().gdn_cuda_release_memory(int(device)))
 
 
 def t10_tables() -> Tables:

@@ -125,6 +125,29 @@ static cudaError_t make_pool(int dev, cudaMemPool_t *pool)
 	return e;
 }
 
+// the current device's pool gives its free memory back
+static cudaError_t trim_pool()
+{
+	int dev = 0;
+	cudaError_t e = cudaGetDevice(&dev);
+	if (e != cudaSuccess)
+		return e;
+	DevMem *m = nullptr;
+	std::lock_guard<std::mutex> g(g_mem_mu);
+	e = mem_of(dev, &m);
+	return e == cudaSuccess && m->pool ? cudaMemPoolTrimTo(m->pool, 0) : e;
+}
+
+cudaError_t dev_malloc(void **p, size_t bytes)
+{
+	cudaError_t e = cudaMalloc(p, bytes);
+	if (e == cudaErrorMemoryAllocation && trim_pool() == cudaSuccess) {
+		cudaGetLastError();
+		e = cudaMalloc(p, bytes);
+	}
+	return e;
+}
+
 cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t s)
 {
 	int dev = 0;
@@ -133,7 +156,7 @@ cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t s)
 		return e;
 	DevMem *m = nullptr;
 	if (bytes > kPoolBlock) {
-		e = cudaMalloc(p, bytes);
+		e = dev_malloc(p, bytes);
 		if (e != cudaSuccess)
 			return e;
 		std::lock_guard<std::mutex> g(g_mem_mu);
@@ -154,7 +177,12 @@ cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t s)
 			return e;
 		pool = m->pool;
 	}
-	return cudaMallocFromPoolAsync(p, bytes, pool, s);
+	e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+	if (e == cudaErrorMemoryAllocation && trim_pool() == cudaSuccess) {
+		cudaGetLastError();
+		e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+	}
+	return e;
 }
 
 void dev_free(void *p, cudaStream_t s)
@@ -1069,6 +1097,13 @@ extern "C" int gdn_cuda_detach(gdn_cuda_handle *h)
 	return GDN_CUDA_OK;
 }
 
+extern "C" int gdn_cuda_release_memory(int device)
+{
+	GDN_CUDA_TRY(cudaSetDevice(device));
+	GDN_CUDA_TRY(trim_pool());
+	return GDN_CUDA_OK;
+}
+
 // ------------------------------------------------------------ stepping --
 
 // ---- enqueue one time step (no host bookkeeping; capturable) ----
@@ -1810,9 +1845,9 @@ extern "C" int gdn_cuda_save_xdmf(gdn_cuda_handle *h, int instance, const char *
 	std::vector<double> nodes(3 * nq), vals((size_t)m * nq);
 	int *owner = nullptr;
 	double *dv = nullptr;
-	cudaError_t ce = cudaMalloc(&owner, (nq > 0 ? nq : 1) * sizeof(int));
+	cudaError_t ce = dev_malloc(reinterpret_cast<void **>(&owner), (nq > 0 ? nq : 1) * sizeof(int));
 	if (ce == cudaSuccess)
-		ce = cudaMalloc(&dv, ((size_t)m * nq > 0 ? (size_t)m * nq : 1) * sizeof(double));
+		ce = dev_malloc(reinterpret_cast<void **>(&dv), ((size_t)m * nq > 0 ? (size_t)m * nq : 1) * sizeof(double));
 	int rc = ce == cudaSuccess ? GDN_CUDA_OK : gdn_cuda_fail(ce, "save_xdmf: cudaMalloc", __FILE__, __LINE__);
 	if (rc == GDN_CUDA_OK) {
 		const int sk = kin ? kin_state_kind(h) : (h->precision == GDN_CUDA_FP64 ? 0 : 1);
@@ -2047,9 +2082,9 @@ extern "C" int gdn_cuda_eval_data(const gdn_cuda_data *d, long long npts, const 
 	int rc = GDN_CUDA_OK;
 	cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
 	if (e == cudaSuccess)
-		e = cudaMalloc(&xd, (size_t)npts * 3 * sizeof(double));
+		e = dev_malloc(reinterpret_cast<void **>(&xd), (size_t)npts * 3 * sizeof(double));
 	if (e == cudaSuccess)
-		e = cudaMalloc(&wd, (size_t)npts * 6 * sizeof(double));
+		e = dev_malloc(reinterpret_cast<void **>(&wd), (size_t)npts * 6 * sizeof(double));
 	if (e == cudaSuccess)
 		e = cudaMemcpyAsync(xd, xyz, (size_t)npts * 3 * sizeof(double), cudaMemcpyHostToDevice, s);
 	if (e == cudaSuccess) {

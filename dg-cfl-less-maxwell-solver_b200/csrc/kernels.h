@@ -20,11 +20,13 @@ namespace gdn {
 // attach + detach, all cudaMalloc / all in the pool / so: kinetic 64^3 FP32 165 + 16
 // / 187 + 50 / 146 + 10, 40^3 FP64 59 + 10 / 51 + 17 / 43 + 9; RK3 48^3 FP64 with two
 // others alive, detach 4.9 / 9.1 / 2.2.
-// The current device is the block's in both calls.
+// The current device is the block's in both calls.  Where memory runs out, the pool
+// gives back what it keeps before the call fails; dev_malloc is cudaMalloc with that.
 constexpr size_t kPoolKeep = (size_t)1 << 30;
 constexpr size_t kPoolBlock = kPoolKeep / 4;
 cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t s);
 void dev_free(void *p, cudaStream_t s);
+cudaError_t dev_malloc(void **p, size_t bytes);
 
 // A handle holds a batch of independent solves (one or more instances): their
 // meshes are concatenated (elements, faces, boundary faces and P2 nodes of

@@ -199,7 +199,7 @@ struct MbBufs {
 	cudaError_t get(X **out, size_t n)
 	{
 		void *q = nullptr;
-		cudaError_t e = cudaMalloc(&q, (n > 0 ? n : 1) * sizeof(X));
+		cudaError_t e = gdn::dev_malloc(&q, (n > 0 ? n : 1) * sizeof(X));
 		if (e == cudaSuccess)
 			p.push_back(q);
 		*out = reinterpret_cast<X *>(q);

@@ -219,6 +219,14 @@ int gdn_cuda_attach_batch(const gdn_cuda_instance *inst, int ninst,
 
 int gdn_cuda_detach(gdn_cuda_handle *h);
 
+/* No counterpart in the reference.  Handles take their smaller device arrays
+ * from a memory pool, which keeps up to 1 GiB of what detached handles gave
+ * back (so that one attach after another does not pay for mapping it) until the
+ * process ends, the device is reset, or memory runs out in a call of this
+ * library.  This call gives all of it back to CUDA device `device`; handles that
+ * are attached are not touched. */
+int gdn_cuda_release_memory(int device);
+
 /* ---- the path ---------------------------------------------------------- */
 
 /* Replaces dg_solve (src/dg/dg.c:23-30): dg_init_sol_macro on the device,

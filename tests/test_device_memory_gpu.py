@@ -5,6 +5,8 @@ import sys
 
 import pytest
 
+from gdon3d_b200 import capi, kuhn
+
 pytestmark = pytest.mark.gpu
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -39,3 +41,28 @@ print("RESET OK")
 def test_attach_after_a_device_reset():
     r = subprocess.run([sys.executable, "-c", RESET % HERE], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "RESET OK" in r.stdout, r.stdout + r.stderr
+
+
+def _free():
+    import torch
+    return torch.cuda.mem_get_info(0)[0]
+
+
+def test_kept_memory_is_given_back():
+    """After the last detach up to 1 GiB is kept; the release call returns it."""
+    mesh = capi.mesh_build(*kuhn.kuhn_cube(32, 0.1, seed=1))
+
+    def once():
+        s = capi.Solver(mesh, dt=1e-4)  # 0.4 GiB, all in pool blocks
+        s.solve(2)
+        s.close()
+
+    once()  # kernels are loaded with their first launch
+    capi.release_memory()
+    before = _free()
+    once()
+    kept = before - _free()
+    assert 0 < kept <= 1 << 30
+    capi.release_memory()
+    assert _free() == before
+    once()  # and the next attach takes it anew
