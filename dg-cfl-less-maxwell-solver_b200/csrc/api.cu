@@ -715,7 +715,19 @@ static int attach_impl(gdn_cuda_handle *h, const gdn_cuda_mesh *m, const gdn_cud
 		GDN_CUDA_TRY(cudaMemcpyAsync(raw, h->nb, 4 * ne * sizeof(int), cudaMemcpyDeviceToDevice, s));
 		GDN_CUDA_TRY(cudaMemcpyAsync(raw + 4 * ne, h->perm, 4 * ne * sizeof(int), cudaMemcpyDeviceToDevice, s));
 		GDN_TRY(launch_rk3_order(h->e2q, h->einst, raw, raw + 4 * ne, ne, h->pos, h->items, h->nb, h->perm, s));
-		h->launches += 2;
+		// kept where it brings the neighbours of a tile together, else the mesh's order
+		unsigned long long sectors[2], *count = reinterpret_cast<unsigned long long *>(h->result);
+		GDN_TRY(launch_rk3_sectors(raw, raw + 4 * ne, ne, count, s));
+		GDN_TRY(launch_rk3_sectors(h->nb, h->perm, ne, count + 1, s));
+		h->launches += 4;
+		GDN_CUDA_TRY(cudaMemcpyAsync(sectors, count, sizeof(sectors), cudaMemcpyDeviceToHost, s));
+		GDN_CUDA_TRY(cudaStreamSynchronize(s));
+		if (sectors[1] >= sectors[0]) {
+			GDN_TRY(launch_rk3_natural_order(ne, h->pos, h->items, s));
+			h->launches++;
+			GDN_CUDA_TRY(cudaMemcpyAsync(h->nb, raw, 4 * ne * sizeof(int), cudaMemcpyDeviceToDevice, s));
+			GDN_CUDA_TRY(cudaMemcpyAsync(h->perm, raw + 4 * ne, 4 * ne * sizeof(int), cudaMemcpyDeviceToDevice, s));
+		}
 		if (fp64) {
 			double *gt;
 			GDN_TRY(dalloc(h, &gt, 10 * nt));

@@ -94,6 +94,10 @@ template <typename T>
 int prepare_rk3();
 
 int rk3_min_blocks(int precision_fp64, int fact, int variant);
+// the mesh's own order, and the gather sectors of an order (rk3_sectors_kernel) into
+// *count (device)
+int launch_rk3_natural_order(long long ne, int *pos, int *items, cudaStream_t s);
+int launch_rk3_sectors(const int *nb, const int *perm, long long ne, unsigned long long *count, cudaStream_t s);
 // device element order: pos[e] (elements of one vertex-index stencil side by
 // side inside blocks, rk3_order_kernel), its inverse items[k], and the neighbour
 // / permutation rows in
