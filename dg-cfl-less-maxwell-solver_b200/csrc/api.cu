@@ -1,6 +1,8 @@
 // The C-ABI of include/gdon3d_cuda.h: handle life cycle, attach (setup on the
 // device), the time loops, state conversion and norms.  Host orchestration
 // only; the arithmetic is in rk3.cu, kinetic.cu and aux.cu.
+#include <algorithm>
+#include <array>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -245,8 +247,8 @@ struct gdn_cuda_handle {
 	void *k2 = nullptr;
 	void *btrace = nullptr; // [2][3][nbf][6][6] boundary traces of the three stages, by step parity (cur)
 	int cur = 0;
-	int rk3_variant = 0; // stage kernel for fewer (0) / more (1) resident CTAs per SM
-	bool rk3_autotune = true; // pick the variant at attach by timing both
+	int rk3_variant = 0; // stage kernel (launch_rk3_stage)
+	bool rk3_autotune = true; // pick the variant at attach
 	// kinetic, in sweep order (item k = position in the level-sorted list)
 	// f: FP64 (FP64, FP32_REFINE), FP32 or BF16; y: FP64 or FP32; G, rs,
 	// rcoef: FP64 (FP64) or FP32
@@ -542,12 +544,14 @@ static const double RK_A[3] = {0., -5. / 9., -153. / 128.};
 static const double RK_B[3] = {1. / 3., 15. / 16., 8. / 15.};
 static const double RK_C[3] = {0., 1. / 3., 3. / 4.};
 
-// RK3 stage-kernel autotuner: times both work decompositions on the handle's
-// own buffers (contents are irrelevant to the timing; init / set_state
-// rewrite them) and keeps the faster one.  Decisions are cached per
-// (precision, floor(log2 ne)) for the life of the process.
+// RK3 stage-kernel autotuner: times the two register caps of one kernel (the same
+// sums, so a state does not depend on the pick; FP64 with the P2 tables has two
+// kernels, and rk3_fp64_variant chooses) on the handle's own buffers (contents are
+// irrelevant to the timing; init / set_state rewrite them) and keeps the faster one.
+// Decisions are cached per (device, precision, kind of tables, floor(log2 ne)) for
+// the life of the process.
 static std::mutex g_tune_mu;
-static std::map<std::pair<int, int>, int> g_tune;
+static std::map<std::array<int, 4>, int> g_tune;
 
 template <typename T>
 static int autotune_rk3(gdn_cuda_handle *h)
@@ -555,7 +559,7 @@ static int autotune_rk3(gdn_cuda_handle *h)
 	int bucket = 0;
 	while ((2LL << bucket) <= h->ne)
 		bucket++;
-	const std::pair<int, int> key(h->precision, bucket);
+	const std::array<int, 4> key = {h->device, h->precision, 2 * h->rk3_sparse + h->rk3_fact, bucket};
 	{
 		std::lock_guard<std::mutex> g(g_tune_mu);
 		auto it = g_tune.find(key);
@@ -757,7 +761,11 @@ static int attach_impl(gdn_cuda_handle *h, const gdn_cuda_mesh *m, const gdn_cud
 		else
 			GDN_TRY(dalloc(h, reinterpret_cast<float **>(&h->k2), 60 * nt));
 		GDN_CUDA_TRY(cudaMemsetAsync(h->k2, 0, 60 * nt * h->ssize, s));
-		if (h->rk3_autotune) {
+		if (h->rk3_autotune && fp64 && h->rk3_fact) {
+			int l2 = 0;
+			GDN_CUDA_TRY(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, h->device));
+			h->rk3_variant = rk3_fp64_variant(ne, h->num_sms, l2, std::min(sectors[0], sectors[1]));
+		} else if (h->rk3_autotune) {
 			GDN_CUDA_TRY(cudaMemsetAsync(h->w[0], 0, 60 * nt * h->ssize, s));
 			GDN_CUDA_TRY(cudaMemsetAsync(h->btrace, 0, 216 * (nbf > 0 ? nbf : 1) * h->ssize, s));
 			if (fp64)

@@ -85,15 +85,19 @@ void rk3_q4(const gdn_cuda_tables *t, double q4[4][10]);
 void rk3_sym_coeffs(const gdn_cuda_tables *t, double q4_sym[6], double minv_sym[7], double s_sym[5]);
 bool rk3_tables_standard_faces(const gdn_cuda_tables *t);
 
-// variant 0 / 1: the stage kernel compiled for fewer / more resident CTAs per
-// SM (rk3_min_blocks), i.e. more / fewer registers per thread.  With the P2
-// tables rk3_elem_kernel (FP32) or rk3_half_kernel (FP64), else rk3_stage_kernel
+// variant 0 / 1: one kernel compiled for fewer / more resident CTAs per SM
+// (rk3_min_blocks), i.e. more / fewer registers per thread: rk3_elem_kernel (FP32
+// with the P2 tables) or rk3_stage_kernel (other tables).  FP64 with the P2 tables:
+// rk3_stage_kernel / rk3_half_kernel, whose sums round differently
 template <typename T>
 int launch_rk3_stage(const Rk3Params<T> &p, int variant, cudaStream_t s);
 template <typename T>
 int prepare_rk3();
 
 int rk3_min_blocks(int precision_fp64, int fact, int variant);
+// the FP64 kernel for the P2 tables, by the mesh (sectors: launch_rk3_sectors of the
+// order in use) and the device alone
+int rk3_fp64_variant(long long ne, int num_sms, long long l2_bytes, unsigned long long sectors);
 // the mesh's own order, and the gather sectors of an order (rk3_sectors_kernel) into
 // *count (device)
 int launch_rk3_natural_order(long long ne, int *pos, int *items, cudaStream_t s);

@@ -1451,9 +1451,28 @@ static int launch_rk3_elem(const Rk3Params<float> &pin, int variant, cudaStream_
 							   p, nblk, kElemThreads, Rk3Elem::smem, s);
 }
 
-// FP64: variant 0 the stage kernel at 2 CTAs of 6 warps per SM (a mesh that does
-// not fill the GPU has three times the warps: 11^3 0.0307 against 0.0326 ms per
-// step), variant 1 the half kernel (32^3 0.342 / 0.275, 48^3 1.12 / 0.84)
+// FP64: variant 0 the stage kernel at 2 CTAs of 6 warps per SM, variant 1 the half
+// kernel.  Their sums round differently (1e-15), so the choice is a rule on the mesh
+// and the device and no timing.  The stage kernel has three times the warps:
+//   it wins while its CTAs are resident at once, 2 per SM (ms per step, it / half
+//   kernel, Kuhn cubes: 4^3 0.0158 / 0.0185, 10^3 0.0206 / 0.0225, 11^3 (250 tiles)
+//   0.0205 / 0.0246, 12^3 (324) 0.0297 / 0.0267, 17^3 0.058 / 0.048, 24^3 0.151 /
+//   0.113; gmsh 452 tiles 0.0369 / 0.0322);
+//   it wins where the gathers go to memory scattered (more than 24 sectors a
+//   gather, rk3_sectors_kernel, and the state read and the one written beyond L2):
+//   elements numbered at random, 31.5 sectors, 24^3 0.250 / 0.232, 28^3 0.453 /
+//   0.461, 32^3 0.842 / 0.885, 48^3 4.83 / 4.95; 48^3 in blocks of 4 at random, 22.4
+//   sectors, 3.05 / 3.05; in blocks of 16, 1.61 / 1.35; 97 k points triangulated,
+//   19.7 sectors, 1.69 / 1.61.
+int rk3_fp64_variant(long long ne, int num_sms, long long l2_bytes, unsigned long long sectors)
+{
+	const long long tiles = (ne + 31) / 32;
+	if (tiles <= (long long)Rk3Variants<double>::lo * num_sms)
+		return 0;
+	const bool scattered = sectors > 24ull * 4ull * (unsigned long long)tiles;
+	return scattered && 2 * tiles * 1920 * (long long)sizeof(double) > l2_bytes ? 0 : 1;
+}
+
 template <bool METAL>
 static int launch_rk3_fp64(const Rk3Params<double> &pin, int variant, cudaStream_t s)
 {
