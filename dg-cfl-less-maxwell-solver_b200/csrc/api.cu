@@ -374,11 +374,6 @@ static void fill_tables(const gdn_cuda_tables *t, Tables<T> &o)
 			o.MinvP[m][j].x = o.Minv[2 * m][j];
 			o.MinvP[m][j].y = o.Minv[2 * m + 1][j];
 		}
-	double q4[4][10];
-	rk3_q4(t, q4);
-	for (int l = 0; l < 4; l++)
-		for (int j = 0; j < 10; j++)
-			o.Q4[l][j] = (T)q4[l][j];
 	double qs[6], ms[7], ss[5];
 	rk3_sym_coeffs(t, qs, ms, ss);
 	for (int k = 0; k < 5; k++)

@@ -35,42 +35,6 @@ int launch_geometry(const int *e2q, const double *node, long long ne, double *ge
 	return GDN_CUDA_OK;
 }
 
-template <typename T>
-__global__ void convert_kernel(const double *__restrict__ a, T *__restrict__ b, long long n)
-{
-	const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-	if (i < n)
-		b[i] = (T)a[i];
-}
-
-template <typename T>
-int launch_convert(const double *a, T *b, long long n, cudaStream_t s)
-{
-	if (n <= 0)
-		return GDN_CUDA_OK;
-	convert_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a, b, n);
-	GDN_CUDA_TRY(cudaGetLastError());
-	return GDN_CUDA_OK;
-}
-template int launch_convert<float>(const double *, float *, long long, cudaStream_t);
-template int launch_convert<__nv_bfloat16>(const double *, __nv_bfloat16 *, long long, cudaStream_t);
-
-__global__ void widen_kernel_f(const float *__restrict__ a, double *__restrict__ b, long long n)
-{
-	const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-	if (i < n)
-		b[i] = (double)a[i];
-}
-
-int launch_widen(const float *a, double *b, long long n, cudaStream_t s)
-{
-	if (n <= 0)
-		return GDN_CUDA_OK;
-	widen_kernel_f<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a, b, n);
-	GDN_CUDA_TRY(cudaGetLastError());
-	return GDN_CUDA_OK;
-}
-
 __device__ __forceinline__ void node_xyz(const int *e2q, const double *node, long long e, int i, double x[3])
 {
 	const long long q = e2q[e * 10 + i];

@@ -13,9 +13,6 @@ struct KinModel {
 };
 
 int launch_geometry(const int *e2q, const double *node, long long ne, double *geom, int *bad, cudaStream_t s);
-template <typename T>
-int launch_convert(const double *a, T *b, long long n, cudaStream_t s);
-int launch_widen(const float *a, double *b, long long n, cudaStream_t s);
 template <typename S>
 int launch_init_rk3(const int *e2q, const double *node, long long k0, long long ne, const int *items, const Data &d,
 					S *w, cudaStream_t s);

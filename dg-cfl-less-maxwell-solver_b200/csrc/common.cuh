@@ -33,10 +33,9 @@ template <typename T>
 struct Tables {
 	typename Vec2<T>::type MinvP[NQN / 2][NQN];
 	T D[3][NQN][NQN];
-	// Q4[l][j] = 4 int lambda_l phi_j (lambda_l the P1 barycentric basis):
-	// D[k] = G_k (Q4 / 4) with G_k the P1 coefficients of d_k(phi_i)
-	T Q4[4][NQN];
-	// The same Q4 and Minv through their tetrahedral symmetry (rk3_sym_coeffs):
+	// Q4[l][j] = 4 int lambda_l phi_j (lambda_l the P1 barycentric basis; D[k] = G_k
+	// (Q4 / 4) with G_k the P1 coefficients of d_k(phi_i)) and Minv through their
+	// tetrahedral symmetry (rk3_sym_coeffs):
 	// an entry depends only on how its two nodes sit (same vertex, two vertices,
 	// a vertex on / off an edge, same edge, edges sharing a vertex, opposite
 	// edges), so a product needs the vertex sum, the edge sum and the sum over
@@ -194,33 +193,6 @@ __device__ __forceinline__ float inv_norm_eps(float nn)
 	return rsqrtf(nn);
 }
 
-// Upwind Maxwell flux (maxwell_num_flux_upwind, src/models/maxwell.c:152-192):
-// with {w} = (wR + wL)/2, [w] = (wR - wL)/2 and r = 1/(|n| + 1e-16),
-//   F_E = -n x {H} + r n x (n x [E]),   F_H = n x {E} + r n x (n x [H]).
-template <typename T>
-__device__ __forceinline__ void upwind_flux(const T wL[6], const T wR[6], const T n[3], T F[6])
-{
-	const T nn = n[0] * n[0] + n[1] * n[1] + n[2] * n[2];
-	const T r = inv_norm_eps(nn);
-	T Es[3], Hs[3], Ed[3], Hd[3];
-#pragma unroll
-	for (int c = 0; c < 3; c++) {
-		Es[c] = T(0.5) * (wR[c] + wL[c]);
-		Hs[c] = T(0.5) * (wR[3 + c] + wL[3 + c]);
-		Ed[c] = T(0.5) * (wR[c] - wL[c]);
-		Hd[c] = T(0.5) * (wR[3 + c] - wL[3 + c]);
-	}
-	const T nEd = n[0] * Ed[0] + n[1] * Ed[1] + n[2] * Ed[2];
-	const T nHd = n[0] * Hd[0] + n[1] * Hd[1] + n[2] * Hd[2];
-	// n x (n x a) = n (n.a) - |n|^2 a
-	F[0] = -(n[1] * Hs[2] - n[2] * Hs[1]) + r * (n[0] * nEd - nn * Ed[0]);
-	F[1] = -(n[2] * Hs[0] - n[0] * Hs[2]) + r * (n[1] * nEd - nn * Ed[1]);
-	F[2] = -(n[0] * Hs[1] - n[1] * Hs[0]) + r * (n[2] * nEd - nn * Ed[2]);
-	F[3] = (n[1] * Es[2] - n[2] * Es[1]) + r * (n[0] * nHd - nn * Hd[0]);
-	F[4] = (n[2] * Es[0] - n[0] * Es[2]) + r * (n[1] * nHd - nn * Hd[1]);
-	F[5] = (n[0] * Es[1] - n[1] * Es[0]) + r * (n[2] * nHd - nn * Hd[2]);
-}
-
 // A(n) w = (-n x H, n x E): the physical Maxwell flux (the upwind flux with
 // wL = wR = w); used for the kinetic equilibrium q = (A_x w, A_y w, A_z w).
 template <typename T>
@@ -237,29 +209,22 @@ __device__ __forceinline__ void maxwell_A(const T n[3], const T w[6], T out[6])
 // Storage conversions for the state (FP64 / FP32 / BF16 storage).
 template <typename S>
 struct Store;
-// load_l2 bypasses L1 (data written by other SMs during the same launch).
 template <>
 struct Store<double> {
 	typedef double compute;
 	__device__ __forceinline__ static double load(const double *p) { return *p; }
-	__device__ __forceinline__ static double load_l2(const double *p) { return __ldcg(p); }
 	__device__ __forceinline__ static void store(double *p, double v) { *p = v; }
 };
 template <>
 struct Store<float> {
 	typedef float compute;
 	__device__ __forceinline__ static float load(const float *p) { return *p; }
-	__device__ __forceinline__ static float load_l2(const float *p) { return __ldcg(p); }
 	__device__ __forceinline__ static void store(float *p, float v) { *p = v; }
 };
 template <>
 struct Store<__nv_bfloat16> {
 	typedef float compute;
 	__device__ __forceinline__ static float load(const __nv_bfloat16 *p) { return __bfloat162float(*p); }
-	__device__ __forceinline__ static float load_l2(const __nv_bfloat16 *p)
-	{
-		return __bfloat162float(__ushort_as_bfloat16(__ldcg(reinterpret_cast<const unsigned short *>(p))));
-	}
 	__device__ __forceinline__ static void store(__nv_bfloat16 *p, float v) { *p = __float2bfloat16_rn(v); }
 };
 

@@ -381,7 +381,7 @@ struct Rk3Variants<double> {
 // Upwind flux with the halving folded into the face quantities: with
 // s = wR + wL, d = wR - wL, n2 = n / 2 and r2 = r / 2 (r = 1 / |n|),
 //   F_E = -n2 x s_H + r2 (n (n . d_E) - |n|^2 d_E),  F_H = n2 x s_E + r2 (n (n . d_H) - |n|^2 d_H),
-// the flux of upwind_flux (maxwell_num_flux_upwind) up to rounding.
+// the flux of maxwell_num_flux_upwind (src/models/maxwell.c:152-192) up to rounding.
 template <typename T>
 __device__ __forceinline__ void upwind_flux_h(const T wL[6], const T wR[6], const T n[3], T F[6])
 {
