@@ -2,7 +2,6 @@
 // device), the time loops, state conversion and norms.  Host orchestration
 // only; the arithmetic is in rk3.cu, kinetic.cu and aux.cu.
 #include <algorithm>
-#include <array>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -248,7 +247,7 @@ struct gdn_cuda_handle {
 	void *btrace = nullptr; // [2][3][nbf][6][6] boundary traces of the three stages, by step parity (cur)
 	int cur = 0;
 	int rk3_variant = 0; // stage kernel (launch_rk3_stage)
-	bool rk3_autotune = true; // pick the variant at attach
+	bool rk3_auto = true; // the variant by rk3_default_variant
 	// kinetic, in sweep order (item k = position in the level-sorted list)
 	// f: FP64 (FP64, FP32_REFINE), FP32 or BF16; y: FP64 or FP32; G, rs,
 	// rcoef: FP64 (FP64) or FP32
@@ -539,90 +538,6 @@ static const double RK_A[3] = {0., -5. / 9., -153. / 128.};
 static const double RK_B[3] = {1. / 3., 15. / 16., 8. / 15.};
 static const double RK_C[3] = {0., 1. / 3., 3. / 4.};
 
-// RK3 stage-kernel autotuner: times the two register caps of one kernel (the same
-// sums, so a state does not depend on the pick; FP64 with the P2 tables has two
-// kernels, and rk3_fp64_variant chooses) on the handle's own buffers (contents are
-// irrelevant to the timing; init / set_state rewrite them) and keeps the faster one.
-// Decisions are cached per (device, precision, kind of tables, floor(log2 ne)) for
-// the life of the process.
-static std::mutex g_tune_mu;
-static std::map<std::array<int, 4>, int> g_tune;
-
-template <typename T>
-static int autotune_rk3(gdn_cuda_handle *h)
-{
-	int bucket = 0;
-	while ((2LL << bucket) <= h->ne)
-		bucket++;
-	const std::array<int, 4> key = {h->device, h->precision, 2 * h->rk3_sparse + h->rk3_fact, bucket};
-	{
-		std::lock_guard<std::mutex> g(g_tune_mu);
-		auto it = g_tune.find(key);
-		if (it != g_tune.end()) {
-			h->rk3_variant = it->second;
-			return GDN_CUDA_OK;
-		}
-	}
-	Rk3Params<T> p;
-	p.w_in = as<T>(h->w[0]);
-	p.w_out = as<T>(h->w[1]);
-	p.k2 = as<T>(h->k2);
-	p.geom = reinterpret_cast<const T *>(h->geomT);
-	p.nb = h->nb;
-	p.perm = h->perm;
-	p.btrace = as<T>(h->btrace);
-	p.einst = h->einst;
-	p.dt_tab = h->dt_dev;
-	p.ne = h->ne;
-	p.dt = h->hdt[0];
-	p.A = RK_A[1];
-	p.B = RK_B[1];
-	p.stage0 = 0;
-	p.write_k2 = 1;
-	p.sparse = h->rk3_sparse;
-	p.fact = h->rk3_fact;
-	p.num_sms = h->num_sms;
-	p.idx32 = (h->ne + 31) / 32 * 1920 <= 0xffffffffLL;
-	p.l2_ahead = 1;
-	p.bc_metal = h->bc_metal;
-	p.traces = 0;
-	cudaEvent_t ev[2];
-	GDN_CUDA_TRY(cudaEventCreate(&ev[0]));
-	GDN_CUDA_TRY(cudaEventCreate(&ev[1]));
-	float best = 0.f;
-	int pick = 0;
-	int rc = GDN_CUDA_OK;
-	for (int v = 0; v < 2 && rc == GDN_CUDA_OK; v++) {
-		float ms = 0.f;
-		for (int rep = 0; rep < 4 && rc == GDN_CUDA_OK; rep++) { // launch 0 warms up
-			if (rep == 1)
-				cudaEventRecord(ev[0], h->stream);
-			rc = launch_rk3_stage<T>(p, v, h->stream);
-			h->launches++;
-		}
-		if (rc != GDN_CUDA_OK)
-			break;
-		cudaEventRecord(ev[1], h->stream);
-		cudaError_t e = cudaEventSynchronize(ev[1]);
-		if (e == cudaSuccess)
-			e = cudaEventElapsedTime(&ms, ev[0], ev[1]);
-		if (e != cudaSuccess)
-			rc = gdn_cuda_fail(e, "autotune_rk3", __FILE__, __LINE__);
-		if (v == 0 || ms < best) {
-			best = ms;
-			pick = v;
-		}
-	}
-	cudaEventDestroy(ev[0]);
-	cudaEventDestroy(ev[1]);
-	if (rc != GDN_CUDA_OK)
-		return rc;
-	h->rk3_variant = pick;
-	std::lock_guard<std::mutex> g(g_tune_mu);
-	g_tune[key] = pick;
-	return GDN_CUDA_OK;
-}
-
 static int kin_prepare_grids(gdn_cuda_handle *h);
 static int kin_prepare_parts(gdn_cuda_handle *h, const gdn_cuda_mesh *m);
 static int autotune_kin(gdn_cuda_handle *h);
@@ -756,17 +671,10 @@ static int attach_impl(gdn_cuda_handle *h, const gdn_cuda_mesh *m, const gdn_cud
 		else
 			GDN_TRY(dalloc(h, reinterpret_cast<float **>(&h->k2), 60 * nt));
 		GDN_CUDA_TRY(cudaMemsetAsync(h->k2, 0, 60 * nt * h->ssize, s));
-		if (h->rk3_autotune && fp64 && h->rk3_fact) {
+		if (h->rk3_auto) {
 			int l2 = 0;
 			GDN_CUDA_TRY(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, h->device));
-			h->rk3_variant = rk3_fp64_variant(ne, h->num_sms, l2, std::min(sectors[0], sectors[1]));
-		} else if (h->rk3_autotune) {
-			GDN_CUDA_TRY(cudaMemsetAsync(h->w[0], 0, 60 * nt * h->ssize, s));
-			GDN_CUDA_TRY(cudaMemsetAsync(h->btrace, 0, 216 * (nbf > 0 ? nbf : 1) * h->ssize, s));
-			if (fp64)
-				GDN_TRY(autotune_rk3<double>(h));
-			else
-				GDN_TRY(autotune_rk3<float>(h));
+			h->rk3_variant = rk3_default_variant(fp64, h->rk3_fact, ne, h->num_sms, l2, std::min(sectors[0], sectors[1]));
 		}
 	} else {
 		const int nv = h->nv;
@@ -1028,7 +936,7 @@ static int attach_batch(const gdn_cuda_instance *inst, int n, const gdn_cuda_tab
 	// RK3 stage kernel compiled for fewer (1) or more (2) resident CTAs per
 	// SM; 0 = timed at attach
 	h->rk3_variant = cfg.rk3_variant > 0 ? cfg.rk3_variant - 1 : 0;
-	h->rk3_autotune = cfg.rk3_variant == 0;
+	h->rk3_auto = cfg.rk3_variant == 0;
 	h->kin_mode = cfg.kin_sweep == 0 ? 1 : cfg.kin_sweep;
 	h->kin_autotune = cfg.kin_sweep == 0;
 	h->ninst = n;
@@ -1408,6 +1316,7 @@ static int kin_first_sweep(gdn_cuda_handle *h, long long &nl)
 // buffers (their contents do not change the work; init / set_state rewrite
 // them) and keeps the faster.  Cached per (precision, floor(log2 items),
 // floor(log2 levels)) for the life of the process.
+static std::mutex g_tune_mu;
 static std::map<std::pair<int, int>, int> g_tune_kin;
 
 static std::pair<int, int> kin_tune_key(const gdn_cuda_handle *h)

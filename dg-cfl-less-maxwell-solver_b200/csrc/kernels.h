@@ -76,7 +76,7 @@ struct Rk3Params {
 	int tile_blocks; // CTAs of the tiles, before those of tr (set at launch)
 	Rk3Trace<T> tr;
 	int idx32; // every tiled state offset fits 32 bits (ntiles * 1920 < 2^32)
-	int l2_ahead; // nonzero: prefetch into L2 the tile this many CTAs ahead (set per variant at launch)
+	int l2_ahead; // nonzero: prefetch into L2 the tile this many tiles ahead (set per variant at launch)
 };
 
 bool rk3_tables_sparse(const gdn_cuda_tables *t);
@@ -95,9 +95,9 @@ template <typename T>
 int prepare_rk3();
 
 int rk3_min_blocks(int precision_fp64, int fact, int variant);
-// the FP64 kernel for the P2 tables, by the mesh (sectors: launch_rk3_sectors of the
-// order in use) and the device alone
-int rk3_fp64_variant(long long ne, int num_sms, long long l2_bytes, unsigned long long sectors);
+// the variant for a mesh (sectors: launch_rk3_sectors of the order in use) on a device
+int rk3_default_variant(int precision_fp64, int fact, long long ne, int num_sms, long long l2_bytes,
+						unsigned long long sectors);
 // the mesh's own order, and the gather sectors of an order (rk3_sectors_kernel) into
 // *count (device)
 int launch_rk3_natural_order(long long ne, int *pos, int *items, cudaStream_t s);

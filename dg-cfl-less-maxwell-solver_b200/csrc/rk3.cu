@@ -16,8 +16,8 @@
 // upwind flux is antisymmetric under (wL, wR, n) -> (wR, wL, -n), so this is
 // the reference's +/- pair up to rounding.  Boundary neighbours read the
 // analytic data at the face-node coordinates and the stage time
-// (dg_update_boundary, dg.c:76-106), written by boundary_trace_kernel just
-// before the stage.
+// (dg_update_boundary, dg.c:76-106), in tables that the step before wrote
+// (rk3_trace_block).
 //
 // Device layout: the state, k2 and the geometry are stored in tiles of 32
 // elements, value-major inside a tile (rk3_tix), elements in the order of
@@ -26,8 +26,8 @@
 // the P1 basis (d(phi_i) is linear) and the products with Q4, S and Minv through
 // their symmetry (rk3_tables_factor):
 //   FP32  rk3_elem_kernel: a thread per element;
-//   FP64  rk3_half_kernel: a thread per element and half (E or H), or on meshes
-//         that do not fill the GPU rk3_stage_kernel (FACT).
+//   FP64  rk3_half_kernel: a thread per element and half (E or H), or where more
+//         warps count (rk3_default_variant) rk3_stage_kernel (FACT).
 // Other tables run rk3_stage_kernel too, a CTA of 6 warps per tile:
 //   0  every thread starts the gathers of its 24 neighbour-trace values
 //      (face node jj = warp of the 4 faces), asynchronously into its own flux
@@ -362,7 +362,7 @@ struct Rk3Smem {
 	static constexpr int bytes_fact = 144 * P * (int)sizeof(T);
 };
 
-// The two autotuned variants of rk3_stage_kernel: register cap (minimum
+// The two variants of rk3_stage_kernel: register cap (minimum
 // resident CTAs per SM) and how the neighbour traces are prefetched (rk3_tile).
 // FP32 runs it only for tables without the P2 symmetry.
 template <typename T>
@@ -370,7 +370,10 @@ struct Rk3Variants;
 template <>
 struct Rk3Variants<float> {
 	static constexpr int lo = 4, hi = 5;
-	static constexpr int pf_lo = 0, pf_hi = 0; // PF_NONE: the pair layout has no constant field stride
+	// PF_NONE: with PF_ASYNC and the flux in packed pairs the best variant is no faster
+	// (ms per step, so / with them: 11^3 0.0217 / 0.0221, 27^3 0.125 / 0.129, 48^3
+	// 0.633 / 0.637; every table entry used: 0.0230 / 0.0230, 0.134 / 0.136, 0.682 / 0.676)
+	static constexpr int pf_lo = 0, pf_hi = 0;
 };
 template <>
 struct Rk3Variants<double> {
@@ -696,18 +699,19 @@ __global__ void __launch_bounds__(kRk3Threads, MINB) rk3_stage_kernel(Rk3Params<
 // all six fields of its element reads every value once, and the (E_c, H_c) pairs
 // of the layout make every step of the residual, which treats E and H alike,
 // packed FP32x2 arithmetic (the flux, the face mass, the derivatives, the lift
-// and the update): 64-bit rows instead of 32-bit ones, 2,250 instead of 6,670
+// and the update): 64-bit rows instead of 32-bit ones, 2,100 instead of 6,670
 // warp instructions and 720 instead of 1,784 L1 wavefronts per tile and stage.
 // The neighbour traces (72 pairs) are copied into the lane's own slots of shared
 // memory asynchronously, a group per face: they are in flight while the curl is
 // computed and hold no register.  k2 stays in registers (copying it too: 2.64 ms
-// per 96^3 step against 2.34).  It is bound by DRAM: 8 warps per SM at 188
-// registers reach 90 % of the copy bandwidth at 96^3; 12 warps at 168 registers
-// spill and reach 84 %.  ms per step, rk3_stage_kernel at 7 launches / this kernel
+// per 96^3 step against 2.34).  It is bound by DRAM: 8 warps per SM at 182
+// registers reach 88 % of the copy bandwidth at 96^3 by the bytes of its own
+// (600 values, 30 of the geometry and 96 bytes of connectivity per element and
+// step); 12 warps at 168 registers spill.  ms per step, rk3_stage_kernel at 7 launches / this kernel
 // at 3: 27^3 0.125 / 0.074, 48^3 0.556 / 0.306, 96^3 4.27 / 2.33.
 constexpr int kElemThreads = 128;
 struct Rk3Elem {
-	static constexpr int lo = 2, hi = 3; // CTAs per SM: 188 / 168 registers
+	static constexpr int lo = 2, hi = 3; // CTAs per SM: 182 / 168 registers
 	static constexpr int smem = kElemThreads / 32 * 72 * 256;
 };
 
@@ -972,12 +976,11 @@ __global__ void __launch_bounds__(kElemThreads, MINB) rk3_elem_kernel(Rk3Params<
 // shared memory, as in rk3_elem_kernel; P then takes their place.
 // rk3_stage_kernel is bound by L1 wavefronts (3,755 per tile and stage, 79 % of
 // the pipe) with FP64 arithmetic at a third of its rate.  ms per step, it / this
-// kernel, both on the reordered elements: 32^3 0.301 / 0.257, 48^3 0.93 / 0.787
-// (4.3 TB/s of the bytes that DRAM moves).  What is left is latency: 254 registers
-// leave 8 warps per SM.
+// kernel, both on the reordered elements: 24^3 0.151 / 0.113, 48^3 0.93 / 0.763.
+// What is left is latency: 254 registers leave 8 warps per SM.
 constexpr int kHalfThreads = 64;
 struct Rk3Half {
-	static constexpr int ctas = 4; // per SM: 255 registers
+	static constexpr int ctas = 4; // per SM: 254 registers
 	static constexpr int smem = 2 * 72 * 32 * (int)sizeof(double);
 };
 
@@ -1424,9 +1427,10 @@ static int launch_rk3_one(const Rk3Params<T> &pin, int variant, cudaStream_t s)
 	typedef Rk3Variants<T> V;
 	Rk3Params<T> p = pin;
 	// L2 prefetch distance: the CTAs resident on the GPU at this variant's cap
-	// (FP32), half of them (FP64).  96^3 ms per step, FP32 / FP64, for none,
-	// half, one and two times the resident CTAs: 4.35 / 9.45, 4.25 / 9.03,
-	// 4.24 / 9.14, 4.32 / 9.67.
+	// (FP32), half of them (FP64).  Chosen when this kernel ran the P2 tables in both
+	// precisions, in the mesh's own order: 96^3 ms per step, FP32 / FP64, for none,
+	// half, one and two times the resident CTAs: 4.35 / 9.45, 4.25 / 9.03, 4.24 /
+	// 9.14, 4.32 / 9.67.
 	const int resident = p.num_sms * (variant == 0 ? V::lo : V::hi);
 	p.l2_ahead = p.l2_ahead ? (sizeof(T) == 8 ? resident / 2 : resident) : 0;
 	const unsigned nblk = (unsigned)((p.ne + 31) / 32);
@@ -1451,28 +1455,8 @@ static int launch_rk3_elem(const Rk3Params<float> &pin, int variant, cudaStream_
 							   p, nblk, kElemThreads, Rk3Elem::smem, s);
 }
 
-// FP64: variant 0 the stage kernel at 2 CTAs of 6 warps per SM, variant 1 the half
-// kernel.  Their sums round differently (1e-15), so the choice is a rule on the mesh
-// and the device and no timing.  The stage kernel has three times the warps:
-//   it wins while its CTAs are resident at once, 2 per SM (ms per step, it / half
-//   kernel, Kuhn cubes: 4^3 0.0158 / 0.0185, 10^3 0.0206 / 0.0225, 11^3 (250 tiles)
-//   0.0205 / 0.0246, 12^3 (324) 0.0297 / 0.0267, 17^3 0.058 / 0.048, 24^3 0.151 /
-//   0.113; gmsh 452 tiles 0.0369 / 0.0322);
-//   it wins where the gathers go to memory scattered (more than 24 sectors a
-//   gather, rk3_sectors_kernel, and the state read and the one written beyond L2):
-//   elements numbered at random, 31.5 sectors, 24^3 0.250 / 0.232, 28^3 0.453 /
-//   0.461, 32^3 0.842 / 0.885, 48^3 4.83 / 4.95; 48^3 in blocks of 4 at random, 22.4
-//   sectors, 3.05 / 3.05; in blocks of 16, 1.61 / 1.35; 97 k points triangulated,
-//   19.7 sectors, 1.69 / 1.61.
-int rk3_fp64_variant(long long ne, int num_sms, long long l2_bytes, unsigned long long sectors)
-{
-	const long long tiles = (ne + 31) / 32;
-	if (tiles <= (long long)Rk3Variants<double>::lo * num_sms)
-		return 0;
-	const bool scattered = sectors > 24ull * 4ull * (unsigned long long)tiles;
-	return scattered && 2 * tiles * 1920 * (long long)sizeof(double) > l2_bytes ? 0 : 1;
-}
-
+// FP64 with the P2 tables: variant 0 the stage kernel at 2 CTAs of 6 warps per SM,
+// variant 1 the half kernel
 template <bool METAL>
 static int launch_rk3_fp64(const Rk3Params<double> &pin, int variant, cudaStream_t s)
 {
@@ -1513,6 +1497,42 @@ int rk3_min_blocks(int precision_fp64, int fact, int variant)
 	if (fact)
 		return variant == 0 ? Rk3Elem::lo : Rk3Elem::hi;
 	return variant == 0 ? Rk3Variants<float>::lo : Rk3Variants<float>::hi;
+}
+
+// The variant by the mesh and the device alone: FP64 has two kernels with the P2
+// tables, whose sums round differently (1e-15), so that a timing would make equal
+// calls give different bits; and a timing of small stages measures their launches
+// (FP32 16^3 took variant 1: 0.0266 ms per step against 0.0219).
+// Figures are ms per step of variant 0 / 1; "sectors" a gather's (rk3_sectors_kernel).
+//   FP32, P2 tables: 0.  3^3 0.0146 / 0.0155, 16^3 0.0219 / 0.0266, 27^3 0.0739 / 0.0782,
+//     96^3 2.64 / 2.73; gmsh 14 k elements 0.0246 / 0.0342, 97 k points triangulated
+//     0.70 / 1.58, 48^3 numbered at random 1.92 / 4.06 (12 warps per SM crowd one
+//     another out of L1 where their gathers touch many sectors).
+//   FP64, P2 tables: 1, but 0 while its CTAs are resident at once, for its three times
+//     as many warps (4^3 0.0158 / 0.0185, 11^3, 250 tiles, 0.0205 / 0.0246, 12^3, 324,
+//     0.0297 / 0.0267, 24^3 0.151 / 0.113; gmsh 452 tiles 0.0369 / 0.0322), and 0 where
+//     the gathers go to memory scattered, i.e. over more than 24 sectors of 32 with the
+//     state read and the one written beyond L2 (numbered at random, 31.5 sectors: 24^3
+//     0.250 / 0.232, 28^3 0.453 / 0.461, 48^3 4.83 / 4.95; 48^3 in blocks of 4 at
+//     random, 22.4, 3.42 / 3.51, of 16, 16.1, 1.92 / 1.86; 97 k points triangulated,
+//     19.7, 1.69 / 1.61).
+//   Other tables: 1, but 0 while its CTAs are resident at once and where a gather takes
+//     more than 10 sectors.  FP64 11^3 0.0237 / 0.0309, 12^3 0.0366 / 0.0328, 27^3, 8.4
+//     sectors, 0.237 / 0.205, 48^3 in blocks of 64 at random, 10.6, 1.45 / 1.69, at
+//     random 4.95 / 8.97; FP32 14^3, 515 tiles, 0.0261 / 0.0299, 16^3, 768, 0.0361 /
+//     0.0360, 27^3 0.134 / 0.127, at random 28^3 0.233 / 0.261.
+int rk3_default_variant(int precision_fp64, int fact, long long ne, int num_sms, long long l2_bytes,
+						unsigned long long sectors)
+{
+	const long long tiles = (ne + 31) / 32;
+	const unsigned long long gathers = 4ull * (unsigned long long)tiles;
+	if (!precision_fp64 && fact)
+		return 0;
+	if (tiles <= (long long)(precision_fp64 ? Rk3Variants<double>::lo : Rk3Variants<float>::lo) * num_sms)
+		return 0;
+	if (!fact)
+		return sectors > 10 * gathers ? 0 : 1;
+	return sectors > 24 * gathers && 2 * tiles * 1920 * (long long)sizeof(double) > l2_bytes ? 0 : 1;
 }
 
 // Device element order.  The neighbour traces of a warp are one access to the

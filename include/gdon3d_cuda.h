@@ -127,14 +127,12 @@ typedef struct gdn_cuda_config {
 	                      per transport solve, 0 to 4 */
 	int rk3_variant; /* RK3 stage kernel.  FP64 with the P2 tables: 1 = a warp
 	                    per field, 2 = a warp per half (E or H), two kernels
-	                    whose sums round differently, 0 = chosen by the mesh and
-	                    the device alone (equal calls give equal bits; a batch
-	                    may run another one than its instances alone).  FP32,
-	                    and tables without the P2 symmetry: 1 = compiled for
-	                    fewer resident CTAs per SM (more registers per thread),
-	                    2 = for more, with the same bits, 0 = the faster of the
-	                    two, timed at attach and cached per (device, precision,
-	                    kind of tables, mesh-size bucket) */
+	                    whose sums round differently.  FP32, and tables without
+	                    the P2 symmetry: 1 = compiled for fewer resident CTAs
+	                    per SM (more registers per thread), 2 = for more, with
+	                    the same bits.  0 = chosen by the mesh and the device
+	                    alone, so that equal calls give equal bits (a batch may
+	                    run another FP64 kernel than its instances alone) */
 	int use_graph; /* capture step loops as CUDA graphs (1 = yes) */
 	int device; /* CUDA device ordinal */
 	int kin_sweep; /* kinetic transport solve: 1 = a launch per sweep level,

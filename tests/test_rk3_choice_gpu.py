@@ -90,3 +90,23 @@ def test_register_caps_give_the_same_bits(precision, tables, bc):
         out.append(s.solve(9)[0])
         s.close()
     assert np.array_equal(out[0], out[1])
+
+
+def _other_tables():
+    t = capi.tables_as_numpy(capi.t10_tables())
+    t["internal"][1][0][0] += 1e-6
+    return capi.tables_from_numpy(t)
+
+
+@pytest.mark.parametrize("n,shuffle", [(2, False), (10, False), (13, False), (18, False), (26, False), (26, True)])
+@pytest.mark.parametrize("precision,other", [(capi.FP32, False), (capi.FP32, True), (capi.FP64, True)])
+def test_no_kernel_is_chosen_by_timing(n, shuffle, precision, other):
+    """FP32 takes the larger register budget with the P2 tables.  Other tables take
+    it while its CTAs are resident at once and where gathers are scattered."""
+    mesh = _mesh(n, shuffle)
+    tiles = (mesh.nbelems + 31) // 32
+    want = 1 if not other or shuffle or tiles <= (2 if precision == capi.FP64 else 4) * _sms() else 2
+    kw = dict(precision=precision, tables=_other_tables() if other else None)
+    variant, launches = _attach(mesh, **kw)
+    assert variant == want
+    assert launches == _attach(mesh, rk3_variant=want, **kw)[1]
