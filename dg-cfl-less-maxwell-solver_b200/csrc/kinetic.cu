@@ -1297,8 +1297,10 @@ __global__ void __launch_bounds__(SweepCfg<T>::threads)
 // lowest level always has its inputs and a warp at work on it: the solve
 // progresses, and its critical path is the longest upwind chain, not the level
 // count times a launch.
-// Registers: 5 CTAs per SM fit at 96 (FP32) and 128 (FP64), 4 with an
-// accumulator (128).
+// Registers: 5 CTAs per SM fit at 96 (FP32) and 128 (FP64), 4 with an accumulator
+// (128).  FP64 is launched at 4 (kin_flow_grid); compiled for 4 it has more registers
+// and no gain (ms per step 4^3 d3q6 0.0946 / 0.0950, 17^3 0.460 / 0.460, 40^3 1.829 /
+// 1.831).
 template <typename F, typename Y, typename T, int ACC, bool BD, bool SPARSE>
 __global__ void __launch_bounds__(SweepCfg<T>::threads, sizeof(T) == 8 || ACC == 0 ? 5 : 4)
 	kin_flow_kernel(KinSweepParams p, const int2 *__restrict__ groups, int ngroups, const int *__restrict__ list,
@@ -1604,10 +1606,10 @@ int kin_flow_grid(int device, int acc, int sparse, int *grid)
 			 : acc == 1 ? (const void *)kin_flow_kernel<F, Y, T, 1, true, false>
 						: (const void *)kin_flow_kernel<F, Y, T, 2, false, false>;
 	GDN_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, SweepCfg<T>::threads, 0));
-	// 16 to 20 warps per SM hold one to two levels of a large mesh; more only
-	// poll, fewer leave a level in parts (ms per step for 2, 3, 4, 5 CTAs per SM:
-	// 64^3 FP32 4.46, 3.93, 3.79, 3.62; 40^3 FP64 2.00, 1.93, 1.94, 1.94, before
-	// the polls below were thinned out)
+	// FP32 20 warps per SM, FP64 12 (4 CTAs of 3): with fewer a level is taken in
+	// parts, more only poll (ms per step, FP64 4 / 5 CTAs: 17^3 0.460 / 0.466, 32^3
+	// 1.164 / 1.177, 40^3 1.829 / 1.825; 64^3 FP32 for 2, 3, 4, 5, before the polls of
+	// warp_gather_wait were thinned out: 4.46, 3.93, 3.79, 3.62)
 	const int cap = sizeof(T) == 4 ? 5 : 4;
 	*grid = nsm * (per > cap ? cap : (per > 0 ? per : 1));
 	return GDN_CUDA_OK;
@@ -1655,7 +1657,7 @@ template int launch_kin_sweep<__nv_bfloat16, float, float>(const KinSweepParams 
 template int launch_kin_sweep<double, float, float>(const KinSweepParams &, int, int, int, cudaStream_t);
 
 // FP64 residual of the transport system of every item (no level order: it
-// only reads y), same thread layout as the sweep:
+// only reads y), a lane per item and a warp per field:
 //   r = f - y - coef Minv (V y + sum_outflow s E S E^T y + sum_inflow s E S tr)
 // with V_ij = -(u . D_ij), u_k = v . codtau[:, k], tr the upwind neighbour's
 // y or the boundary f_eq.  This is f - b - M1 y with M1 as the blocks kernel
