@@ -322,8 +322,8 @@ def main():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--variant", type=int, default=0, choices=[0, 1, 2],
-                    help="RK3 stage kernel: 1 / 2 = compiled for fewer / more resident CTAs per SM, "
-                         "0 = autotuned")
+                    help="RK3 stage kernel: variant 1 or 2 (rk3_variant of gdn_cuda_config), "
+                         "0 = chosen by the attach")
     ap.add_argument("--only", default="all",
                     help="profiling aid: comma-separated variants to run (rk3: fp64,fp32; kinetic: "
                          "fp64,fp32,fp32_refine1,fp32_refine2,bf16)")

@@ -580,9 +580,8 @@ __device__ __forceinline__ void store10(S *p, const T v[10])
 // G is read by its six lanes at one address (broadcast), one wavefront per
 // 16 bytes; a warp shares nothing with other warps, so there is no CTA barrier.
 // ms per step before (lane = item, 32 items per CTA) and after, the fastest
-// grouping of each (jittered meshes, d3q4): 17^3 FP64 0.76 / 0.43, 24^3 FP32 with
-// one refinement 3.03 / 1.38, 40^3 FP64 2.83 / 1.73, 64^3 FP32 5.83 / 3.62; a
-// level of 457 items takes 2.4 us (4.4 before), of 9250 items 3.5 us (7.4).
+// grouping of each (jittered meshes, d3q4): 17^3 FP64 0.76 / 0.46, 24^3 FP32 with
+// one refinement 3.03 / 1.40, 40^3 FP64 2.83 / 1.83, 64^3 FP32 5.83 / 3.71.
 constexpr int kSwSlots = 5; // items per warp
 
 // Warps per CTA (static shared memory below 48 KB) and items per CTA.
@@ -939,8 +938,8 @@ __device__ __forceinline__ void warp_gather(const KinSweepParams &p, const Sweep
 // and is ready when it is not "unwritten".  Nothing else passes between the CTAs,
 // so no flag, fence or ordering between the values of a row is needed.  (Rows copied
 // by cp.async are not atomic by the memory model; ms per step with them / as here:
-// 17^3 FP64 0.428 / 0.457, 40^3 FP64 1.73 / 1.82, 40^3 FP32 1.23 / 1.25, 64^3 FP32
-// 3.64 / 3.66.  A fence and a flag per warp: 17^3 0.67, 64^3 4.4.)
+// 17^3 FP64 0.424 / 0.461, 40^3 FP64 1.73 / 1.83, 40^3 FP32 1.23 / 1.28, 64^3 FP32
+// 3.62 / 3.71.  FP64 traces straight from L2: 17^3 0.511, 40^3 2.18.  A fence and a flag per warp: 17^3 0.67, 64^3 4.4.)
 // One lane per row polls the row's last value until it is written; then the rows
 // are fetched, and polled on should a trace still be missing.  Most warps are
 // ahead of their inputs, so what waiting costs the others counts: lanes leave the

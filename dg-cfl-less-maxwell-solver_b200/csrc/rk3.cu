@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(kRk3Threads, MINB) rk3_stage_kernel(Rk3Params<
 // memory asynchronously, a group per face: they are in flight while the curl is
 // computed and hold no register.  k2 stays in registers (copying it too: 2.64 ms
 // per 96^3 step against 2.34).  It is bound by DRAM: 8 warps per SM at 182
-// registers reach 88 % of the copy bandwidth at 96^3 by the bytes of its own
+// registers reach 90 % of the copy bandwidth at 96^3 by the bytes of its own
 // (600 values, 30 of the geometry and 96 bytes of connectivity per element and
 // step); 12 warps at 168 registers spill.  ms per step, rk3_stage_kernel at 7 launches / this kernel
 // at 3: 27^3 0.125 / 0.074, 48^3 0.556 / 0.306, 96^3 4.27 / 2.33.
